@@ -95,7 +95,10 @@ struct AvgDesc {
 cudaError_t gba_launch_avg_finish(const AvgDesc& d, int64_t rows, int sms, cudaStream_t s);
 
 size_t gba_preagg_smem_bytes(const QDesc& q, int S, int T, int nstages, int use_tma);
-cudaError_t gba_launch_table_init(const GTable& t, const QDesc& q, int grid, cudaStream_t s);
+// cap: device word holding the table's slot count when the host does not know it (else t.cap)
+cudaError_t gba_launch_table_init(const GTable& t, const QDesc& q, int grid, cudaStream_t s,
+                                  const unsigned long long* cap = nullptr);
 cudaError_t gba_launch_preagg(const QDesc& q, const GTable& t, const PreaggCfg& c, unsigned* flags,
                               cudaStream_t s);
-cudaError_t gba_launch_compact(const GTable& t, const QDesc& q, const OutDesc& o, int grid, cudaStream_t s);
+cudaError_t gba_launch_compact(const GTable& t, const QDesc& q, const OutDesc& o, int grid, cudaStream_t s,
+                               const unsigned long long* cap = nullptr);

@@ -322,7 +322,9 @@ __device__ __forceinline__ void init_slots(const GTable& t, int naccs, const uns
   }
 }
 
-__global__ void k_table_init(GTable t, int naccs, QDesc q) {
+// cap: when set, the table's slots as a kernel before this one decided them
+__global__ void k_table_init(GTable t, int naccs, QDesc q, const unsigned long long* cap) {
+  if (cap) t.cap = *cap;
   unsigned long long id[GBA_MAX_AGGS];
 #pragma unroll
   for (int a = 0; a < GBA_MAX_AGGS; ++a) id[a] = a < naccs ? acc_identity(q.acc_op[a]) : 0ull;
@@ -399,7 +401,9 @@ __device__ __forceinline__ void compact_side(const GTable& t, const QDesc& q, co
     if (a < q.naccs) o.accs[a][pos] = side[1 + a];
 }
 
-__global__ void __launch_bounds__(kCompactThreads) k_compact(GTable t, QDesc q, OutDesc o) {
+__global__ void __launch_bounds__(kCompactThreads) k_compact(GTable t, QDesc q, OutDesc o,
+                                                             const unsigned long long* cap) {
+  if (cap) t.cap = *cap;
   for (uint64_t lo = uint64_t(blockIdx.x) * kCompactSlots; lo < t.cap; lo += uint64_t(gridDim.x) * kCompactSlots)
     compact_range(t, q, o, lo, lo + kCompactSlots < t.cap ? lo + kCompactSlots : t.cap);
   if (blockIdx.x == 0 && threadIdx.x == 0) compact_side(t, q, o);
@@ -481,8 +485,9 @@ size_t gba_preagg_smem_bytes(const QDesc& q, int S, int T, int nstages, int use_
   return b;
 }
 
-cudaError_t gba_launch_table_init(const GTable& t, const QDesc& q, int grid, cudaStream_t s) {
-  k_table_init<<<grid, 256, 0, s>>>(t, q.naccs, q);
+cudaError_t gba_launch_table_init(const GTable& t, const QDesc& q, int grid, cudaStream_t s,
+                                  const unsigned long long* cap) {
+  k_table_init<<<grid, 256, 0, s>>>(t, q.naccs, q, cap);
   return cudaGetLastError();
 }
 
@@ -509,8 +514,9 @@ cudaError_t gba_launch_preagg(const QDesc& q, const GTable& t, const PreaggCfg& 
   });
 }
 
-cudaError_t gba_launch_compact(const GTable& t, const QDesc& q, const OutDesc& o, int grid, cudaStream_t s) {
-  k_compact<<<grid, kCompactThreads, 0, s>>>(t, q, o);
+cudaError_t gba_launch_compact(const GTable& t, const QDesc& q, const OutDesc& o, int grid, cudaStream_t s,
+                               const unsigned long long* cap) {
+  k_compact<<<grid, kCompactThreads, 0, s>>>(t, q, o, cap);
   return cudaGetLastError();
 }
 

@@ -2,61 +2,74 @@
 #pragma once
 #include "gba_kernels.h"
 
-// One histogram/scatter work unit: a run of rows inside one input segment.
-struct PartChunk {
-  int64_t row_begin, row_end;
-  int64_t count_base;  // first counts[] entry of the chunk's segment
-  int seg_nchunks;     // chunks in that segment
-  int chunk_in_seg;
+// A run of rows of one hot partition (too many rows for one CTA): its groups
+// are merged in the HBM fallback table.
+struct PartPiece {
+  long long row_begin, row_end;
 };
 
-// One MSD partition pass over `bits` hash bits below the `shift_hi` bits
-// already used.  counts/offsets layout: [segment][digit][chunk-in-segment].
+// What the plan kernel tells the kernels after it (device memory).
+struct PartPlan {
+  unsigned long long fb_cap;  // slots of the fallback table
+  int npieces;
+  int pad;
+};
+
+// k_part_plan: from the 2^(bits1 + bits2) partition counts to bounds.
+struct PartPlanArgs {
+  int bits1, bits2;  // digit bits of the two passes (bits2 = 0: one pass)
+  const unsigned long long* hist;
+  unsigned long long* offs;      // first row of every partition, then n
+  unsigned long long* cursors1;  // write cursors of the first pass
+  unsigned long long* cursors2;  // of the second pass
+  unsigned* tile_prefix;         // second pass: first tile of every first-pass segment, then all tiles
+  int tile2;                     // rows per tile of the second pass
+  int64_t hot_rows, piece_rows;  // partitions of more than hot_rows rows are cut into pieces
+  PartPiece* pieces;
+  int max_pieces;
+  unsigned long long fb_cap, fb_per_hot;  // fallback slots, plus those per hot partition
+  PartPlan* plan;
+};
+
+// One partition pass over `bits` hash bits below the `shift_hi` bits already
+// used.  nseg = 0: the rows [0, n) are one segment; else the segments are the
+// first pass's partitions, segment s starting at offs[s << bits].
 struct PartPass {
   QDesc in;   // rows read (keys + value columns)
   QDesc out;  // rows written (keys + value columns, same types)
-  const PartChunk* chunks;
-  int nchunks;
-  int shift_hi;
-  int bits;
-  unsigned* counts;
-  const unsigned long long* offsets;
-};
-
-// One work item of the final aggregation: whole partitions [seg_lo, seg_hi),
-// or (partial = 1) the rows [row_begin, row_end) of one partition too large
-// for one CTA; a partial piece merges its groups into the HBM table.
-struct PartWork {
-  int seg_lo, seg_hi;
-  int partial;
-  int pad;
-  int64_t row_begin, row_end;
+  int64_t n;
+  int shift_hi, bits;
+  int nseg;
+  int T;                        // rows per tile (<= gba_part_scatter_max_tile())
+  int threads;                  // 512 (two CTAs per SM) or 1024 (one)
+  const unsigned long long* offs;
+  const unsigned* tile_prefix;  // nseg + 1 entries
+  unsigned long long* cursors;  // [segment][digit]
+  unsigned* flags;
 };
 
 // Final aggregation: one shared-memory table per partition (or piece).
 struct PartAgg {
-  QDesc rows;                 // partitioned rows + aggregate spec
-  const long long* seg_begin; // nsegs + 1 entries
-  int nsegs;
-  const PartWork* work;       // work items, largest first
-  int nwork;
-  unsigned* seg_ctr;          // dynamic work queue (zeroed before launch)
-  int S;                      // shared table slots
-  int sprobe;
-  int coalesce;
-  GTable fallback;            // keys whose probe window is full + pieces of split partitions
+  QDesc rows;                      // partitioned rows + aggregate spec
+  const unsigned long long* offs;  // nparts + 1 entries
+  int nparts;
+  const PartPiece* pieces;
+  const PartPlan* plan;
+  int64_t hot_rows;
+  unsigned* ctr;                   // dynamic work queue (zeroed before launch)
+  int S;                           // shared table slots (whole 16-byte buckets)
+  int nbk;                         // buckets probed before a row goes to the fallback table
+  GTable fallback;                 // keys whose probe window is full + pieces (its cap: plan->fb_cap)
   unsigned* flags;
   OutDesc out;
 };
 
-size_t gba_part_scatter_smem(const QDesc& q, int bits, int T);
-cudaError_t gba_launch_part_hist(const PartPass& p, int grid, cudaStream_t s);
-cudaError_t gba_launch_scan_excl(const unsigned* in, unsigned long long* out, int64_t n,
-                                 unsigned long long* status, unsigned* tile_ctr, unsigned* flags, cudaStream_t s);
-cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, int T, cudaStream_t s);
-// seg_begin[s * 2^bits + d] = offsets[count_base[s] + d * seg_nchunks[s]] for
-// every input segment s; seg_begin[nseg_in * 2^bits] = total rows
-cudaError_t gba_launch_seg_begins(const unsigned long long* offsets, const long long* count_base,
-                                  const int* seg_nchunks, int nseg_in, int bits, int64_t total,
-                                  long long* seg_begin, cudaStream_t s);
-cudaError_t gba_launch_part_agg(const PartAgg& a, int grid, cudaStream_t s);
+size_t gba_part_scatter_smem(const QDesc& q, int bits, int nseg, int T);
+int gba_part_scatter_max_tile();
+// shared table slots of k_part_agg with 2 or 3 CTAs per SM
+int gba_part_agg_slots(const QDesc& q, int ctas, int max_smem_optin);
+size_t gba_part_agg_smem(const QDesc& q, int S);
+cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* hist, int sms, cudaStream_t s);
+cudaError_t gba_launch_part_plan(const PartPlanArgs& a, cudaStream_t s);
+cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s);
+cudaError_t gba_launch_part_agg(const PartAgg& a, int ctas, int grid, cudaStream_t s);

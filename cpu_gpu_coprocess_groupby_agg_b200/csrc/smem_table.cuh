@@ -200,8 +200,6 @@ __device__ __forceinline__ unsigned long long smem_acc_read(const SmemTable<K64>
   return __double_as_longlong(d);
 }
 
-// init all slots (called by the whole CTA; caller syncs): every accumulator
-// word starts at its op's identity (fixed-point words and residual at 0)
 // Merges every group of a shared table into an HBM table (all threads of the
 // block; the caller syncs before and after).
 template <bool K64, typename Sig>
@@ -223,37 +221,47 @@ __device__ __forceinline__ void smem_flush_to_gtable(const QDesc& q, const GTabl
   }
 }
 
+// slot i back to empty: every accumulator word at its op's identity
+// (fixed-point words and residual at 0)
 template <bool K64, typename Sig>
-__device__ __forceinline__ void smem_table_init(const SmemTable<K64>& t, const QDesc& q) {
-  for (int i = threadIdx.x; i < t.S; i += blockDim.x) {
-    t.keys[i] = smem_empty_key<K64>();
+__device__ __forceinline__ void smem_slot_reset(const SmemTable<K64>& t, const QDesc& q, int i) {
+  t.keys[i] = smem_empty_key<K64>();
 #pragma unroll
-    for (int a = 0; a < Sig::NA; ++a) {
-      const int op = Sig::op(q, a), w = Sig::woff(q, a);
-      const AccRef r = smem_ref<K64>(t, w, i);
-      if (op == ACC_MIN_I || op == ACC_MAX_I) {
-        *r.w64 = acc_identity(op);
-      } else if (op == ACC_CNT) {
-        *r.lo = 0u;
-      } else {
-        *r.lo = 0u;
-        *r.hi = 0u;
-        if (op == ACC_ADD_F) {
-          const AccRef r1 = smem_ref<K64>(t, w + 2, i);
-          *r1.lo = 0u;
-          *r1.hi = 0u;
-          *smem_ref<K64>(t, w + 4, i).w64 = 0ull;
-        }
+  for (int a = 0; a < Sig::NA; ++a) {
+    const int op = Sig::op(q, a), w = Sig::woff(q, a);
+    const AccRef r = smem_ref<K64>(t, w, i);
+    if (op == ACC_MIN_I || op == ACC_MAX_I) {
+      *r.w64 = acc_identity(op);
+    } else if (op == ACC_CNT) {
+      *r.lo = 0u;
+    } else {
+      *r.lo = 0u;
+      *r.hi = 0u;
+      if (op == ACC_ADD_F) {
+        const AccRef r1 = smem_ref<K64>(t, w + 2, i);
+        *r1.lo = 0u;
+        *r1.hi = 0u;
+        *smem_ref<K64>(t, w + 4, i).w64 = 0ull;
       }
     }
   }
-  if (threadIdx.x == 0) {
-    for (int w = 0; w < Sig::nwords(q); ++w) t.side()[w] = 0ull;
+}
+
+// the all-ones key's side slot back to absent (one thread)
+template <bool K64, typename Sig>
+__device__ __forceinline__ void smem_side_reset(const SmemTable<K64>& t, const QDesc& q) {
+  for (int w = 0; w < Sig::nwords(q); ++w) t.side()[w] = 0ull;
 #pragma unroll
-    for (int a = 0; a < Sig::NA; ++a)
-      if (Sig::op(q, a) != ACC_ADD_F) t.side()[Sig::woff(q, a)] = acc_identity(Sig::op(q, a));
-    *t.side_present() = 0u;
-  }
+  for (int a = 0; a < Sig::NA; ++a)
+    if (Sig::op(q, a) != ACC_ADD_F) t.side()[Sig::woff(q, a)] = acc_identity(Sig::op(q, a));
+  *t.side_present() = 0u;
+}
+
+// empties the whole table (called by the whole CTA; caller syncs)
+template <bool K64, typename Sig>
+__device__ __forceinline__ void smem_table_init(const SmemTable<K64>& t, const QDesc& q) {
+  for (int i = threadIdx.x; i < t.S; i += blockDim.x) smem_slot_reset<K64, Sig>(t, q, i);
+  if (threadIdx.x == 0) smem_side_reset<K64, Sig>(t, q);
 }
 
 // Warp-cooperative coalescing of equal keys (all 32 lanes call it).  Lanes
