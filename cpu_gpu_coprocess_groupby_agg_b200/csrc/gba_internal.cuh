@@ -60,6 +60,16 @@ __device__ __forceinline__ uint32_t fast_hash(uint64_t k, uint64_t mul) {
 __device__ __forceinline__ uint32_t table_hash(uint64_t k) { return fast_hash(k, 0x9e3779b97f4a7c15ull); }
 __device__ __forceinline__ uint32_t part_hash(uint64_t k) { return fast_hash(k, 0xd6e8feb86659fd93ull); }
 
+// Place of k among 2^bits - 1 ascending splitters: how many are <= k.
+__device__ __forceinline__ unsigned gba_range_digit(const unsigned long long* split, int bits, unsigned long long k) {
+  unsigned pos = 0;
+  for (int b = bits - 1; b >= 0; --b) {
+    const unsigned mid = pos + (1u << b);
+    pos = split[mid - 1] <= k ? mid : pos;
+  }
+  return pos;
+}
+
 // ---------------------------------------------------------------------------
 // Row access.
 __device__ __forceinline__ uint64_t load_key_g(const QDesc& q, int64_t r) {

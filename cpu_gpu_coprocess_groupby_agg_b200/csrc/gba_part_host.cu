@@ -48,6 +48,22 @@ size_t row_bytes(const QDesc& q) {
 
 }  // namespace
 
+// Rows per tile: two CTAs of 512 threads per SM, each with two tiles of rows in
+// flight; where a digit's run in such a tile would be under 24 rows, one CTA of
+// 1024 threads with larger tiles (measured, two CTAs against one: 2^28 rows of
+// 24 bytes in 7 + 8 bits 5.73 against 5.03 ms; 2^27 rows of 16 bytes in 6 + 7
+// bits 1.64 against 2.09 ms).
+int gba_part_tile_rows(const QDesc& q, int bits, int nseg, bool range, int max_smem_optin, int* threads) {
+  auto fit = [&](size_t budget) {
+    int T = gba_part_scatter_max_tile();
+    while (T > 512 && gba_part_scatter_smem(q, bits, nseg, T, range) > budget) T -= 256;
+    return T;
+  };
+  const int T = fit(size_t(max_smem_optin) / 2 - 1536);
+  *threads = T >> bits < 24 && T < gba_part_scatter_max_tile() ? 1024 : 512;
+  return *threads == 512 ? T : fit(size_t(max_smem_optin) - 1536);
+}
+
 int gba_choose_strategy(const gba_context* ctx, const QDesc& q, const gba_knobs& k, double predicted_groups,
                         const GbaPlan& p) {
   (void)k;
@@ -97,23 +113,9 @@ gba_status gba_run_partition(gba_context* ctx, const QDesc& q, const gba_output*
     const int b1 = B <= kOnePassBits ? B : B / 2, b2 = B - b1;
     ctx->stats.partition_bits = B;
     const int64_t nparts = int64_t(1) << B;
-    // Rows per tile: two CTAs of 512 threads per SM, each with two tiles of
-    // rows in flight; where a digit's run in such a tile would be under 24 rows,
-    // one CTA of 1024 threads with larger tiles (measured, two CTAs against
-    // one: 2^28 rows of 24 bytes in 7 + 8 bits 5.73 against 5.03 ms; 2^27 rows
-    // of 16 bytes in 6 + 7 bits 1.64 against 2.09 ms).
-    auto tile_rows = [&](int bits, int nseg, int* threads) {
-      auto fit = [&](size_t budget) {
-        int T = gba_part_scatter_max_tile();
-        while (T > 512 && gba_part_scatter_smem(q, bits, nseg, T) > budget) T -= 256;
-        return T;
-      };
-      const int T = fit(size_t(ctx->max_smem_optin) / 2 - 1536);
-      *threads = T >> bits < 24 && T < gba_part_scatter_max_tile() ? 1024 : 512;
-      return *threads == 512 ? T : fit(size_t(ctx->max_smem_optin) - 1536);
-    };
     int th1 = 512, th2 = 512;
-    const int T1 = tile_rows(b1, 0, &th1), T2 = b2 > 0 ? tile_rows(b2, 1 << b1, &th2) : 0;
+    const int T1 = gba_part_tile_rows(q, b1, 0, false, ctx->max_smem_optin, &th1);
+    const int T2 = b2 > 0 ? gba_part_tile_rows(q, b2, 1 << b1, false, ctx->max_smem_optin, &th2) : 0;
     const uint64_t fb_cap = std::max<uint64_t>(1 << 16, uint64_t(std::min<double>(groups * 0.02, 1 << 24)));
 
     Carver cv;

@@ -211,8 +211,11 @@ __device__ __forceinline__ void stage_ends(unsigned char* dst, const unsigned ch
 // unless there are 2^32 rows).  THREADS: 512 (two CTAs per SM, one's copies
 // and barriers behind the other's work) or 1024 (one CTA with tiles of twice
 // the rows, for passes whose runs would be short).
-template <bool K64, int NC, typename IdxT, int THREADS>
+// RANGE: the digit is the key's place among the segment's splitters (the
+// key-ordered output, k_sort.cu) instead of bits of its hash.
+template <bool K64, int NC, typename IdxT, int THREADS, bool RANGE>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPass p) {
+  if (RANGE && *p.fail) return;  // the whole grid: set by an earlier kernel
   constexpr int kScatterThreads = THREADS;
   constexpr int kScatterRpt = kScatterRows / THREADS;
   extern __shared__ __align__(16) unsigned char sm[];
@@ -226,6 +229,12 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPa
   unsigned* hist = lofs + nb;
   unsigned* segs = hist + nb;  // second pass: tile prefix of the segments
   unsigned* order = segs + (p.nseg > 0 ? p.nseg + 2 : 0);
+  unsigned long long* split = nullptr;  // RANGE: the current segment's splitters
+  if (RANGE) {
+    split = reinterpret_cast<unsigned long long*>((reinterpret_cast<uintptr_t>(order) + 7) & ~uintptr_t(7));
+    order = reinterpret_cast<unsigned*>(split + nb);
+  }
+  int split_seg = -1;
   unsigned char* buf0 = reinterpret_cast<unsigned char*>(order + T);
   buf0 = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(buf0) + 15) & ~uintptr_t(15));
   __shared__ unsigned wsum[kScatterThreads / 32];
@@ -331,6 +340,11 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPa
     for (int c = 0; c < NC; ++c)
       scol[c] = src + coff[c] + ((reinterpret_cast<uintptr_t>(p.in.cols[c]) + size_t(r0) * cw[c]) & 15);
     const int nrows = rows;
+    if (RANGE && split_seg != seg) {  // (uniform over the CTA)
+      split_seg = seg;
+      for (int i = tid; i < nb; i += kScatterThreads) split[i] = p.splitters[(size_t(seg) << p.bits) + i];
+      __syncthreads();
+    }
     unsigned long long* cursors = p.cursors + (size_t(seg) << (p.nseg > 0 ? p.bits : 0));
     if (tile + gridDim.x < ntiles) {
       locate(tile + gridDim.x, r0, rows, seg);
@@ -343,7 +357,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPa
       const int j = i * kScatterThreads + tid;
       dr[i] = 0;
       if (j < nrows) {
-        const unsigned d = digit_of(skey[j], p.shift_hi, p.bits);
+        const unsigned d = RANGE ? gba_range_digit(split, p.bits, skey[j] ^ KeyT(p.flip))
+                                 : digit_of(skey[j], p.shift_hi, p.bits);
         dr[i] = d << 16 | atomicAdd(&hist[d], 1u);
       }
     }
@@ -803,9 +818,9 @@ __global__ void __launch_bounds__(kAggThreads, MINB) k_part_agg(PartAgg a) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-size_t gba_part_scatter_smem(const QDesc& q, int bits, int nseg, int T) {
+size_t gba_part_scatter_smem(const QDesc& q, int bits, int nseg, int T, bool range) {
   const size_t nb = size_t(1) << bits;
-  size_t b = nb * (8 + 4 + 4) + (nseg > 0 ? size_t(nseg + 2) * 4 : 0) + size_t(T) * 4 + 16;
+  size_t b = (range ? nb * 8 + 8 : 0) + nb * (8 + 4 + 4) + (nseg > 0 ? size_t(nseg + 2) * 4 : 0) + size_t(T) * 4 + 16;
   auto col = [&](size_t w) { return ((size_t(T) * w + 15) & ~size_t(15)) + 16; };
   size_t rows = col(q.key64 ? 8 : 4);
   for (int c = 0; c < q.ncols; ++c) rows += col(gba_type_bytes(q.col_type[c]));
@@ -857,28 +872,39 @@ cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s)
   // the kernel's digit scan takes at most two digits per thread
   if (p.bits < 1 || (1 << p.bits) > 1024 || p.T > kScatterRows || (p.threads != 512 && p.threads != 1024))
     return cudaErrorInvalidValue;
-  const size_t smem = gba_part_scatter_smem(p.in, p.bits, p.nseg, p.T);
+  const size_t smem = gba_part_scatter_smem(p.in, p.bits, p.nseg, p.T, p.splitters != nullptr);
   auto go = [&](auto kernel) -> cudaError_t {
     cudaError_t e = gba_allow_max_smem(kernel);
     if (e != cudaSuccess) return e;
     kernel<<<grid, p.threads, smem, s>>>(p);
     return cudaGetLastError();
   };
-  auto cols = [&](auto K, auto I) -> cudaError_t {
-    constexpr bool k64 = decltype(K)::value;
+  auto shape = [&](auto K, auto I, auto N, auto R) -> cudaError_t {
+    constexpr bool k64 = decltype(K)::value, range = decltype(R)::value;
+    constexpr int nc = decltype(N)::value;
     using IdxT = decltype(I);
+    return p.threads == 1024 ? go(k_part_scatter<k64, nc, IdxT, 1024, range>)
+                             : go(k_part_scatter<k64, nc, IdxT, 512, range>);
+  };
+  auto cols = [&](auto K, auto I, auto R) -> cudaError_t {
     switch (p.in.ncols) {
-      case 0: return p.threads == 1024 ? go(k_part_scatter<k64, 0, IdxT, 1024>) : go(k_part_scatter<k64, 0, IdxT, 512>);
-      case 1: return p.threads == 1024 ? go(k_part_scatter<k64, 1, IdxT, 1024>) : go(k_part_scatter<k64, 1, IdxT, 512>);
-      case 2: return p.threads == 1024 ? go(k_part_scatter<k64, 2, IdxT, 1024>) : go(k_part_scatter<k64, 2, IdxT, 512>);
-      case 3: return p.threads == 1024 ? go(k_part_scatter<k64, 3, IdxT, 1024>) : go(k_part_scatter<k64, 3, IdxT, 512>);
-      case 4: return p.threads == 1024 ? go(k_part_scatter<k64, 4, IdxT, 1024>) : go(k_part_scatter<k64, 4, IdxT, 512>);
+      case 0: return shape(K, I, std::integral_constant<int, 0>{}, R);
+      case 1: return shape(K, I, std::integral_constant<int, 1>{}, R);
+      case 2: return shape(K, I, std::integral_constant<int, 2>{}, R);
+      case 3: return shape(K, I, std::integral_constant<int, 3>{}, R);
+      case 4: return shape(K, I, std::integral_constant<int, 4>{}, R);
     }
     return cudaErrorInvalidValue;
   };
   const bool wide = p.n >= (int64_t(1) << 32);
-  if (p.in.key64) return wide ? cols(std::true_type{}, 0ull) : cols(std::true_type{}, 0u);
-  return wide ? cols(std::false_type{}, 0ull) : cols(std::false_type{}, 0u);
+  const std::true_type yes{};
+  const std::false_type no{};
+  if (p.splitters) {
+    if (wide) return cudaErrorInvalidValue;
+    return p.in.key64 ? cols(yes, 0u, yes) : cols(no, 0u, yes);
+  }
+  if (p.in.key64) return wide ? cols(yes, 0ull, no) : cols(yes, 0u, no);
+  return wide ? cols(no, 0ull, no) : cols(no, 0u, no);
 }
 
 cudaError_t gba_launch_part_agg(const PartAgg& a, int ctas, int grid, cudaStream_t s) {

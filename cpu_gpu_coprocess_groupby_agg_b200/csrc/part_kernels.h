@@ -46,6 +46,12 @@ struct PartPass {
   const unsigned* tile_prefix;  // nseg + 1 entries
   unsigned long long* cursors;  // [segment][digit]
   unsigned* flags;
+  // digits by key range (key-ordered output) instead of by hash: 2^bits - 1
+  // splitters per segment ([segment][2^bits] words) of keys ^ flip; the pass is
+  // skipped when *fail is set
+  const unsigned long long* splitters;
+  unsigned long long flip;
+  const unsigned* fail;
 };
 
 // Final aggregation: one shared-memory table per partition (or piece).
@@ -64,7 +70,9 @@ struct PartAgg {
   OutDesc out;
 };
 
-size_t gba_part_scatter_smem(const QDesc& q, int bits, int nseg, int T);
+size_t gba_part_scatter_smem(const QDesc& q, int bits, int nseg, int T, bool range = false);
+// rows per tile of a pass, and its CTA shape (threads)
+int gba_part_tile_rows(const QDesc& q, int bits, int nseg, bool range, int max_smem_optin, int* threads);
 int gba_part_scatter_max_tile();
 // shared table slots of k_part_agg with 2 or 3 CTAs per SM
 int gba_part_agg_slots(const QDesc& q, int ctas, int max_smem_optin);

@@ -26,6 +26,6 @@ inline SortJob gba_sort_job(const gba_query* q, const gba_output* out, int64_t g
   return j;
 }
 
-// Sorts every job's groups, one job after another on stream s, in the context
-// workspace; one host round trip for all jobs' key ranges and one at the end.
+// Sorts every job's groups on stream s, in the context workspace; one host
+// round trip at the end (more only where the sample sort does not apply).
 gba_status gba_sort_groups(gba_context* ctx, const SortJob* jobs, int njobs, cudaStream_t s);
