@@ -702,8 +702,32 @@ static gba_status groupby_device(gba_context* ctx, const gba_query* q, const gba
     if (st != GBA_OK) return st;
     ctx->stats.predicted_groups = pred;
   }
+  return gba_run_planned(ctx, qd, out, k, pred, s, n_groups);
+}
+
+// Plans and runs a query whose estimate (learned sizing; else -1) is known.
+gba_status gba_run_planned(gba_context* ctx, const QDesc& qd, const gba_output* out, const gba_knobs& k, double pred,
+                           cudaStream_t s, int64_t* n_groups) {
   GbaPlan p;
   gba_make_plan(ctx, qd, k, pred, &p);
+  if (gba_sample_wanted(qd, k)) {
+    double groups = 0;
+    bool few = false;
+    int counted_bits = 0;
+    gba_status st = gba_sample_groups(ctx, qd, k, gba_table_groups(ctx, qd), s, &groups, &few, &counted_bits);
+    if (st != GBA_OK) return st;
+    if (!few) return gba_run_partition(ctx, qd, out, k, p, groups, s, n_groups, counted_bits);
+    // a table for 32 times the sampled groups; should even that overflow, the
+    // rows are partitioned by their count
+    p.table_slots = std::min(p.table_slots, gba_pow2_ceil(uint64_t(std::max(65536.0, 32.0 * groups))));
+    gba_knobs once = k;
+    once.max_regrow = 0;
+    st = gba_run_table(ctx, qd, out, once, p, s, n_groups);
+    if (st != GBA_ERR_TABLE_OVERFLOW) return st;
+    ctx->err.clear();
+    ctx->stats.regrows++;
+    return gba_run_partition(ctx, qd, out, k, p, -1.0, s, n_groups);
+  }
   int strategy = k.strategy;
   if (strategy == GBA_STRATEGY_AUTO) strategy = gba_choose_strategy(ctx, qd, k, pred, p);
   if (strategy == GBA_STRATEGY_PARTITION) return gba_run_partition(ctx, qd, out, k, p, pred, s, n_groups);

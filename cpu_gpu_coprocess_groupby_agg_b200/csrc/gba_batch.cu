@@ -682,10 +682,29 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
     ipre[j + 1] = ipre[j] + int64_t(std::max<size_t>(1, (words + 256 * 16 - 1) / (256 * 16)));
     cpre[j + 1] = cpre[j] + int64_t(std::max<uint64_t>(1, (x.p.table_slots + 2047) / 2048));
   }
-  if (nt > 0) {
+  // partition-strategy queries: a status block each behind the tables, then
+  // one workspace that they use one after another (with kernel timing on they
+  // run one by one after the launch instead, each with its own times)
+  std::vector<int> pq;
+  for (int i = 0; i < nq && k.timing == 0; ++i)
+    if (qi[i].strategy == GBA_STRATEGY_PARTITION) pq.push_back(i);
+  const size_t npq = pq.size();
+  const size_t o_pstat = take(GBA_PART_STATUS * std::max<size_t>(npq, 1));
+  std::vector<PartShape> psh(npq);
+  size_t part_bytes = 0;
+  int part_launches = 0;
+  for (size_t x = 0; x < npq; ++x) {
+    size_t b = 0;
+    gba_part_shape(ctx, qd[pq[x]], k, pred[pq[x]], &psh[x]);
+    gba_part_enqueue(ctx, qd[pq[x]], &outs[pq[x]], psh[x], qi[pq[x]].p.smem_probe_cap, nullptr, &b, nullptr, nullptr,
+                     &part_launches, s);
+    part_bytes = std::max(part_bytes, b);
+  }
+  const size_t o_part = take(part_bytes);
+  if (nt > 0 || npq > 0) {
     gba_status st = gba_ws_reserve(ctx, off, s);
     if (st != GBA_OK) return st;
-    st = gba_batch_host_reserve(ctx, desc_bytes + stat_bytes + 256);
+    st = gba_batch_host_reserve(ctx, round_up(desc_bytes, 256) + round_up(stat_bytes, 256) + GBA_PART_STATUS * npq + 256);
     if (st != GBA_OK) return st;
   }
   unsigned char* d = static_cast<unsigned char*>(ctx->ws);
@@ -806,6 +825,24 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
     GBA_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
     for (auto& ev : ctx->fork_ev) GBA_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
+  const size_t h_pstat = h_stat + round_up(stat_bytes, 256);
+  if (npq > 0) {
+    GBA_CUDA_TRY(ctx, cudaMemsetAsync(d + o_pstat, 0, GBA_PART_STATUS * npq, s));
+    for (size_t x = 0; x < npq; ++x) {
+      size_t b = 0;
+      const int i = pq[x];
+      gba_status st = gba_part_enqueue(ctx, qd[i], &outs[i], psh[x], qi[i].p.smem_probe_cap, d + o_part, &b,
+                                       d + o_pstat + GBA_PART_STATUS * x, nullptr, &part_launches, s);
+      if (st != GBA_OK) return st;
+    }
+    GBA_CUDA_TRY(ctx, cudaMemcpyAsync(h + h_pstat, d + o_pstat, GBA_PART_STATUS * npq, cudaMemcpyDeviceToHost, s));
+    if (nt == 0) GBA_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    ctx->stats.kernel_launches += part_launches;
+    for (int i : pq) {
+      ctx->stats.main_rows += qd[i].n;
+      ctx->stats.main_bytes += qd[i].n * int64_t(gba_row_bytes(qd[i]));
+    }
+  }
   if (nt > 0) {
     for (int g = 0; g < ng; ++g)
       GBA_CUDA_TRY(ctx, groups[g].tma ? gba_prepare_stream_tma(groups[g].proto, groups[g].cluster, groups[g].shape)
@@ -914,6 +951,29 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
       result = GBA_ERR_OUTPUT_CAPACITY;
     }
   }
+  std::vector<char> done(nq, 0);
+  for (size_t x = 0; x < npq; ++x) {
+    const int i = pq[x];
+    const unsigned flags = *reinterpret_cast<const unsigned*>(h + h_pstat + GBA_PART_STATUS * x);
+    const unsigned long long cnt = *reinterpret_cast<const unsigned long long*>(h + h_pstat + GBA_PART_STATUS * x + 8);
+    if (flags & GBA_FLAG_WAIT_TIMEOUT) {
+      ctx->err = "query " + std::to_string(i) + ": a bounded wait for a staged tile timed out";
+      return GBA_ERR_TIMEOUT;
+    }
+    if (flags & GBA_FLAG_TABLE_OVERFLOW) {  // an under-estimate: rerun alone with more partitions, below
+      acc.regrows++;
+      qi[i].pred *= 4.0;
+      continue;
+    }
+    done[i] = 1;
+    acc.partition_bits = std::max(acc.partition_bits, psh[x].bits);
+    n_groups[i] = int64_t(cnt);
+    if (int64_t(cnt) > outs[i].capacity && result == GBA_OK) {
+      ctx->err = "query " + std::to_string(i) + ": output capacity " + std::to_string(outs[i].capacity) + " < " +
+                 std::to_string(cnt) + " groups";
+      result = GBA_ERR_OUTPUT_CAPACITY;
+    }
+  }
   auto run_alone = [&](int i) -> gba_status {
     GbaPlan p = qi[i].p;
     gba_status st;
@@ -943,7 +1003,7 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
     }
   }
   for (int i = 0; i < nq; ++i) {
-    if (qi[i].strategy == GBA_STRATEGY_TABLE) continue;
+    if (qi[i].strategy == GBA_STRATEGY_TABLE || done[i]) continue;
     ctx->stats = gba_stats{};
     const gba_status st = run_alone(i);
     if (st != GBA_OK) {

@@ -102,8 +102,7 @@ extern "C" gba_status gba_groupby_host(gba_context* ctx, const gba_query* q, con
       st = stage_all();
       if (st != GBA_OK) return st;
     }
-    st = strategy == GBA_STRATEGY_PARTITION ? gba_run_partition(ctx, dq, &dout, k, p, pred, s, &ng)
-                                            : gba_run_table(ctx, dq, &dout, k, p, s, &ng);
+    st = gba_run_planned(ctx, dq, &dout, k, pred, s, &ng);
   } else {
     // Chunked pipeline: H2D of chunk i+1 overlaps the pre-aggregation of chunk i.
     const int64_t chunk = std::max<int64_t>(int64_t(p.tile_rows), int64_t(1) << 23) / p.tile_rows * p.tile_rows;

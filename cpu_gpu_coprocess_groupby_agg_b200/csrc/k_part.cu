@@ -43,7 +43,7 @@ constexpr int kHistIlp = 8;
 
 template <bool K64>
 __global__ void __launch_bounds__(kHistThreads) k_part_hist(const void* keys, int64_t n, int bits,
-                                                            unsigned long long* hist) {
+                                                            unsigned long long* hist, const unsigned* skip) {
   extern __shared__ unsigned cnt[];
   const int sub = bits < kHistBits ? bits : kHistBits;
   const int nb = 1 << sub;
@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(kHistThreads) k_part_hist(const void* keys, in
   __syncthreads();
   const int64_t step = int64_t(gridDim.x) * (kHistThreads * kHistIlp);
   for (int64_t r0 = int64_t(blockIdx.x) * (kHistThreads * kHistIlp); r0 < n; r0 += step) {
+    // set by the row sample that runs beside this kernel: the counts are not needed
+    if (skip && *reinterpret_cast<const volatile unsigned*>(skip)) break;
     uint64_t k[kHistIlp];
 #pragma unroll
     for (int u = 0; u < kHistIlp; ++u) {
@@ -118,7 +120,9 @@ __global__ void __launch_bounds__(1024) k_part_plan(PartPlanArgs a) {
     unsigned long long c[kPlanPer], sum = 0;
 #pragma unroll
     for (int i = 0; i < kPlanPer; ++i) {
-      c[i] = p0 + i < np ? a.hist[p0 + i] : 0ull;
+      c[i] = 0;
+      if (p0 + i < np)
+        for (int x = 0; x < 1 << a.hist_shift; ++x) c[i] += a.hist[(size_t(p0 + i) << a.hist_shift) + x];
       sum += c[i];
     }
     unsigned long long chunk;
@@ -848,7 +852,8 @@ int gba_part_agg_slots(const QDesc& q, int ctas, int max_smem_optin) {
 
 int gba_part_scatter_max_tile() { return kScatterRows; }
 
-cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* hist, int sms, cudaStream_t s) {
+cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* hist, int sms, const unsigned* skip,
+                                 cudaStream_t s) {
   const int sub = bits < kHistBits ? bits : kHistBits;
   const size_t smem = (size_t(1) << sub) * 4;
   auto go = [&](auto kernel) -> cudaError_t {
@@ -857,7 +862,7 @@ cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* h
     const int64_t want = (q.n + kHistThreads * kHistIlp - 1) / (kHistThreads * kHistIlp);
     const int64_t most = int64_t(sms) * (smem <= 64 * 1024 ? 2 : 1);
     const dim3 grid(unsigned(want < 1 ? 1 : want < most ? want : most), 1u << (bits - sub));
-    kernel<<<grid, kHistThreads, smem, s>>>(q.keys, q.n, bits, hist);
+    kernel<<<grid, kHistThreads, smem, s>>>(q.keys, q.n, bits, hist, skip);
     return cudaGetLastError();
   };
   return q.key64 ? go(k_part_hist<true>) : go(k_part_hist<false>);

@@ -19,6 +19,7 @@ struct PartPlan {
 struct PartPlanArgs {
   int bits1, bits2;  // digit bits of the two passes (bits2 = 0: one pass)
   const unsigned long long* hist;
+  int hist_shift;                // counts per partition: 2^hist_shift consecutive ones
   unsigned long long* offs;      // first row of every partition, then n
   unsigned long long* cursors1;  // write cursors of the first pass
   unsigned long long* cursors2;  // of the second pass
@@ -77,7 +78,9 @@ int gba_part_scatter_max_tile();
 // shared table slots of k_part_agg with 2 or 3 CTAs per SM
 int gba_part_agg_slots(const QDesc& q, int ctas, int max_smem_optin);
 size_t gba_part_agg_smem(const QDesc& q, int S);
-cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* hist, int sms, cudaStream_t s);
+// skip: a device word; once it is set the kernel stops early (null: never)
+cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* hist, int sms, const unsigned* skip,
+                                 cudaStream_t s);
 cudaError_t gba_launch_part_plan(const PartPlanArgs& a, cudaStream_t s);
 cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s);
 cudaError_t gba_launch_part_agg(const PartAgg& a, int ctas, int grid, cudaStream_t s);
