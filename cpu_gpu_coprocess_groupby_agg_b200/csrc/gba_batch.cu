@@ -618,6 +618,13 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
     int64_t first = 0;
     // work-item takers of the launch: CTAs, or clusters of g.cluster CTAs
     const int takers = g.cluster > 1 ? std::max(1, g.grid / g.cluster) : ctx->sms * g.minb;
+    // the rows of a launch of small queries are shared out over all takers,
+    // whatever their merges then cost (48 queries of up to 2^18 rows, us of the
+    // four launches: 910 with items of 16 merges, 204 with one share per taker,
+    // 211 with half a share)
+    int64_t launch_rows = 0;
+    for (int i : order) launch_rows += qd[i].n;
+    const int64_t share = std::max<int64_t>(T, (launch_rows / takers + T - 1) / T * T);
     for (int i : order) {
       int64_t ir = (qd[i].n + takers - 1) / takers;
       // an item ends by merging its shared table into HBM (one insert per
@@ -628,7 +635,7 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
       const int64_t merges =
           qi[i].S > 0 ? int64_t(std::min<double>(qi[i].pred > 0 ? qi[i].pred : tslots, tslots)) : 0;
       ir = std::max<int64_t>(ir, 16 * merges);
-      ir = std::min(item_cap, std::max<int64_t>(T, (ir + T - 1) / T * T));
+      ir = std::min({item_cap, share, std::max<int64_t>(T, (ir + T - 1) / T * T)});
       const int64_t nit = (qd[i].n + ir - 1) / ir;
       if (nit == 0) continue;
       spans.push_back(BatchSpan{qi[i].slot, 0, ir, first});
