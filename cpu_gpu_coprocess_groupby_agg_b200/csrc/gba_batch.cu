@@ -765,10 +765,11 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
   // nodes when captured): [0] table init, [1] pre-aggregation, [2] compaction
   const bool timing = k.timing != 0;
   const bool as_graph = k.use_graph != 0;
+  bool capturing = false;
   auto mark = [&](int i, cudaStream_t cs) -> cudaError_t {
     if (!timing) return cudaSuccess;
     // inside a capture the event record must be an external graph node
-    return as_graph ? cudaEventRecordWithFlags(ctx->tev[i], cs, cudaEventRecordExternal) : cudaEventRecord(ctx->tev[i], cs);
+    return capturing ? cudaEventRecordWithFlags(ctx->tev[i], cs, cudaEventRecordExternal) : cudaEventRecord(ctx->tev[i], cs);
   };
   const int64_t* d_ipre = reinterpret_cast<const int64_t*>(d + o_ipre);
   const int64_t* d_cpre = reinterpret_cast<const int64_t*>(d + o_cpre);
@@ -895,13 +896,21 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
         key.push_back(int64_t(g.smem));
         key.push_back(int64_t(g.members.size()));
       }
-      if (!ctx->batch_exec || key != ctx->batch_key) {
+      // A shape seen for the first time is launched directly: capturing and
+      // instantiating its graph takes about 300 us of host time, its launches
+      // about 40, and batches of new data rarely have the last one's shape
+      // (their tables follow the estimates).  The second time it is captured.
+      const bool replay = ctx->batch_exec && key == ctx->batch_key;
+      const bool capture = !replay && (k.use_graph > 0 || key == ctx->batch_seen);
+      ctx->batch_seen = key;
+      if (capture) {
         if (ctx->batch_exec) {
           cudaGraphExecDestroy(ctx->batch_exec);
           ctx->batch_exec = nullptr;
         }
         if (!ctx->cap_stream) GBA_CUDA_TRY(ctx, cudaStreamCreateWithFlags(&ctx->cap_stream, cudaStreamNonBlocking));
         GBA_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->cap_stream, cudaStreamCaptureModeThreadLocal));
+        capturing = true;
         const cudaError_t e = enqueue(ctx->cap_stream);
         cudaGraph_t graph = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(ctx->cap_stream, &graph);
@@ -912,7 +921,8 @@ static gba_status batch_device(gba_context* ctx, int32_t nq, const gba_query* qs
         GBA_CUDA_TRY(ctx, e3);
         ctx->batch_key = key;
       }
-      GBA_CUDA_TRY(ctx, cudaGraphLaunch(ctx->batch_exec, s));
+      if (ctx->batch_exec && key == ctx->batch_key) GBA_CUDA_TRY(ctx, cudaGraphLaunch(ctx->batch_exec, s));
+      else GBA_CUDA_TRY(ctx, enqueue(s));
     } else {
       GBA_CUDA_TRY(ctx, enqueue(s));
     }

@@ -48,6 +48,7 @@ struct gba_context {
   cudaEvent_t fork_ev[2] = {};
   cudaGraphExec_t batch_exec = nullptr;
   std::vector<int64_t> batch_key;
+  std::vector<int64_t> batch_seen;  // the last shape launched without a graph
   // drop-in API: a tile's groups before the reference-layout partitioning
   void* rp_buf = nullptr;
   size_t rp_bytes = 0;

@@ -145,7 +145,8 @@ typedef struct gba_knobs {
   int32_t smem_probe_cap; /* shared table probe cap (0 = auto) */
   int32_t max_regrow;     /* regrow attempts before GBA_ERR_TABLE_OVERFLOW */
   int32_t timing;         /* 1: time each kernel with CUDA events (gba_stats.kernel_ms) */
-  int32_t use_graph;      /* batch: -1 auto (on), 0 off, 1 on: replay the launch sequence as a CUDA graph */
+  int32_t use_graph;      /* batch: replay the launch sequence as a CUDA graph: -1 auto (once a batch has the
+                             launch shapes of the one before it), 0 off, 1 on */
   int32_t item_rows;      /* batch: rows per work-queue item (0 = auto) */
   double learned_load;    /* learned sizing: HBM table load at the predicted group count (0 = auto: 0.35 for
                              one query, 0.25 in a batch) */
