@@ -70,6 +70,22 @@ __device__ __forceinline__ unsigned gba_range_digit(const unsigned long long* sp
   return pos;
 }
 
+// The same for R keys step by step together, so that their reads overlap.
+template <int R>
+__device__ __forceinline__ void gba_range_digits(const unsigned long long* split, int bits,
+                                                 const unsigned long long (&k)[R], unsigned (&d)[R]) {
+#pragma unroll
+  for (int i = 0; i < R; ++i) d[i] = 0;
+#pragma unroll 1
+  for (int b = bits - 1; b >= 0; --b) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const unsigned mid = d[i] + (1u << b);
+      d[i] = split[mid - 1] <= k[i] ? mid : d[i];
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Row access.
 __device__ __forceinline__ uint64_t load_key_g(const QDesc& q, int64_t r) {

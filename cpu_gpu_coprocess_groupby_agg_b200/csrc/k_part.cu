@@ -218,8 +218,16 @@ __device__ __forceinline__ void stage_ends(unsigned char* dst, const unsigned ch
 // RANGE: the digit is the key's place among the segment's splitters (the
 // key-ordered output, k_sort.cu) instead of bits of its hash.
 template <bool K64, int NC, typename IdxT, int THREADS, bool RANGE>
-__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPass p) {
-  if (RANGE && *p.fail) return;  // the whole grid: set by an earlier kernel
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPass one, const PartPass* many) {
+  // RANGE: pass blockIdx.y of an array
+  __shared__ __align__(8) unsigned char s_pass[RANGE ? sizeof(PartPass) : 8];
+  if (RANGE) {
+    for (int w = threadIdx.x; w < int(sizeof(PartPass) / 4); w += THREADS)
+      reinterpret_cast<unsigned*>(s_pass)[w] = reinterpret_cast<const unsigned*>(many + blockIdx.y)[w];
+    __syncthreads();
+  }
+  const PartPass& p = RANGE ? *reinterpret_cast<const PartPass*>(s_pass) : one;
+  if (RANGE && *p.fail) return;  // the whole pass: set by an earlier kernel
   constexpr int kScatterThreads = THREADS;
   constexpr int kScatterRpt = kScatterRows / THREADS;
   extern __shared__ __align__(16) unsigned char sm[];
@@ -356,13 +364,20 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_part_scatter(PartPa
     }
     // every row's digit and its rank among the tile's rows of that digit
     unsigned dr[kScatterRpt];
+    if constexpr (RANGE) {
+      unsigned long long k[kScatterRpt];
+#pragma unroll
+      for (int i = 0; i < kScatterRpt; ++i) {
+        const int j = i * kScatterThreads + tid;
+        k[i] = j < nrows ? skey[j] ^ KeyT(p.flip) : 0ull;
+      }
+      gba_range_digits<kScatterRpt>(split, p.bits, k, dr);
+    }
 #pragma unroll
     for (int i = 0; i < kScatterRpt; ++i) {
       const int j = i * kScatterThreads + tid;
-      dr[i] = 0;
       if (j < nrows) {
-        const unsigned d = RANGE ? gba_range_digit(split, p.bits, skey[j] ^ KeyT(p.flip))
-                                 : digit_of(skey[j], p.shift_hi, p.bits);
+        const unsigned d = RANGE ? dr[i] : digit_of(skey[j], p.shift_hi, p.bits);
         dr[i] = d << 16 | atomicAdd(&hist[d], 1u);
       }
     }
@@ -873,15 +888,23 @@ cudaError_t gba_launch_part_plan(const PartPlanArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s) {
-  // the kernel's digit scan takes at most two digits per thread
-  if (p.bits < 1 || (1 << p.bits) > 1024 || p.T > kScatterRows || (p.threads != 512 && p.threads != 1024))
-    return cudaErrorInvalidValue;
-  const size_t smem = gba_part_scatter_smem(p.in, p.bits, p.nseg, p.T, p.splitters != nullptr);
+namespace {
+// one pass (many null) or a device array of `n` RANGE passes whose host copies
+// start at &p: all of one key width, column count and CTA shape
+cudaError_t launch_scatter(const PartPass& p, const PartPass* many, int n, int grid, cudaStream_t s) {
+  size_t smem = 0;
+  for (int i = 0; i < n; ++i) {
+    const PartPass& x = (&p)[i];
+    // the kernel's digit scan takes at most two digits per thread
+    if (x.bits < 1 || (1 << x.bits) > 1024 || x.T > kScatterRows || (x.threads != 512 && x.threads != 1024))
+      return cudaErrorInvalidValue;
+    const size_t b = gba_part_scatter_smem(x.in, x.bits, x.nseg, x.T, many != nullptr);
+    smem = b > smem ? b : smem;
+  }
   auto go = [&](auto kernel) -> cudaError_t {
     cudaError_t e = gba_allow_max_smem(kernel);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, p.threads, smem, s>>>(p);
+    kernel<<<dim3(unsigned(grid), unsigned(n)), p.threads, smem, s>>>(p, many);
     return cudaGetLastError();
   };
   auto shape = [&](auto K, auto I, auto N, auto R) -> cudaError_t {
@@ -904,12 +927,20 @@ cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s)
   const bool wide = p.n >= (int64_t(1) << 32);
   const std::true_type yes{};
   const std::false_type no{};
-  if (p.splitters) {
+  if (many) {
     if (wide) return cudaErrorInvalidValue;
     return p.in.key64 ? cols(yes, 0u, yes) : cols(no, 0u, yes);
   }
   if (p.in.key64) return wide ? cols(yes, 0ull, no) : cols(yes, 0u, no);
   return wide ? cols(no, 0ull, no) : cols(no, 0u, no);
+}
+}  // namespace
+
+cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s) {
+  return launch_scatter(p, nullptr, 1, grid, s);
+}
+cudaError_t gba_launch_part_scatter_many(const PartPass* host, const PartPass* device, int n, int grid, cudaStream_t s) {
+  return launch_scatter(*host, device, n, grid, s);
 }
 
 cudaError_t gba_launch_part_agg(const PartAgg& a, int ctas, int grid, cudaStream_t s) {

@@ -22,11 +22,11 @@
 // Bytes per group of b bytes: 2 (b + key) per level and 2 b for the buckets,
 // against 2 (key + 4) for each of up to 8 passes plus the random gather of a
 // least-significant-digit sort over (key, index) pairs.  Measured (us, that
-// sort / this one): 16.8M int64 groups with 2 aggregates 2714 / 1130, 9.9M with
-// 1 aggregate 1390 / 695, 48 queries of up to 2^17 groups (the whole batch
-// call) 5410 / 1590.  The bucket kernel (2.3 TB/s on the 16.8M groups) is bound
-// by its barriers and shared-memory round trips at 3 CTAs of 512 threads per
-// SM (2 CTAs: 500 against 350 us), the count by the binary search's
+// sort / this one): 16.8M int64 groups with 2 aggregates 2714 / 1190, 9.9M with
+// 1 aggregate 1390 / 695; 48 queries of up to 2^17 groups, sorted in one launch
+// per step, 4200 / 90.  The bucket kernel (2.1 TB/s on the 16.8M groups) is
+// bound by its barriers and shared-memory round trips at 3 CTAs of 512 threads
+// per SM (2 CTAs: 500 against 380 us), the count by the binary search's
 // shared-memory reads.
 //
 // Jobs beyond the two levels, and a job with a bucket that outgrows shared
@@ -520,12 +520,28 @@ __device__ __forceinline__ unsigned long long sort_key(const void* keys, int key
          flip;
 }
 
-// splitters of segment blockIdx.x (rows [offs[x], offs[x + 1]), or [0, n) when
-// offs is null) from an evenly spaced sample of its keys
-__global__ void __launch_bounds__(kSampleThreads) k_sort_split(const void* keys, int key64, unsigned long long flip,
-                                                               int64_t n, const unsigned long long* offs, int bits,
-                                                               unsigned long long* split) {
+// All kernels of the sample sort take an array of jobs, one per blockIdx.y.
+struct SortSplitArgs {
+  const void* keys;
+  int key64;
+  unsigned long long flip;
+  int64_t n;
+  int bits, nseg;                  // nseg = 0: one segment [0, n)
+  const unsigned long long* offs;  // segment bounds
+  unsigned long long* split;       // [segment][2^bits]
+};
+
+// splitters of segment blockIdx.x from an evenly spaced sample of its keys
+__global__ void __launch_bounds__(kSampleThreads) k_sort_split(const SortSplitArgs* jobs) {
   extern __shared__ __align__(16) unsigned char sm[];
+  const SortSplitArgs a = jobs[blockIdx.y];
+  if (int(blockIdx.x) >= (a.nseg > 0 ? a.nseg : 1)) return;
+  const void* keys = a.keys;
+  const int key64 = a.key64, bits = a.bits;
+  const unsigned long long flip = a.flip;
+  const int64_t n = a.n;
+  const unsigned long long* offs = a.nseg > 0 ? a.offs : nullptr;
+  unsigned long long* split = a.split;
   const CtaOrder<kSampleCap, kSampleThreads, kSampleBins> s(sm);
   const int64_t b = offs ? int64_t(offs[blockIdx.x]) : 0, e = offs ? int64_t(offs[blockIdx.x + 1]) : n;
   const int64_t rows = e - b;
@@ -555,7 +571,8 @@ struct SortHistArgs {
 
 // A CTA takes consecutive tiles, so it reloads splitters and adds its counts
 // to the segment's once per segment it meets.
-__global__ void __launch_bounds__(512) k_sort_hist(SortHistArgs a) {
+__global__ void __launch_bounds__(512) k_sort_hist(const SortHistArgs* jobs) {
+  const SortHistArgs a = jobs[blockIdx.y];
   __shared__ unsigned long long split[1 << kLevelBits];
   __shared__ unsigned cnt[1 << kLevelBits];
   const int nb = 1 << a.bits, tid = threadIdx.x;
@@ -592,16 +609,22 @@ __global__ void __launch_bounds__(512) k_sort_hist(SortHistArgs a) {
       }
       __syncthreads();
     }
-    for (int64_t r = r0 + tid; r < e; r += 4 * 512) {
-      unsigned long long k[4];
+    const unsigned long long flip = a.flip;
+    const int bits = a.bits, rows = int(e - r0);
+    auto count = [&](auto keys) {
+      for (int r = tid; r < rows; r += 8 * 512) {
+        unsigned long long k[8];
+        unsigned d[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) k[u] = r + u * 512 < e ? sort_key(a.keys, a.key64, r + u * 512, a.flip) : 0ull;
+        for (int u = 0; u < 8; ++u) k[u] = r + u * 512 < rows ? __ldg(keys + r + u * 512) ^ flip : 0ull;
+        gba_range_digits<8>(split, bits, k, d);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const unsigned d = gba_range_digit(split, a.bits, k[u]);
-        if (r + u * 512 < e) atomicAdd(&cnt[d], 1u);
+        for (int u = 0; u < 8; ++u)
+          if (r + u * 512 < rows) atomicAdd(&cnt[d[u]], 1u);
       }
-    }
+    };
+    if (a.key64) count(static_cast<const unsigned long long*>(a.keys) + r0);
+    else count(static_cast<const unsigned*>(a.keys) + r0);
   }
   __syncthreads();
   flush();
@@ -618,7 +641,8 @@ struct SortPlanArgs {
   unsigned* fail;
 };
 
-__global__ void __launch_bounds__(1024) k_sort_plan(SortPlanArgs a) {
+__global__ void __launch_bounds__(1024) k_sort_plan(const SortPlanArgs* jobs) {
+  const SortPlanArgs a = jobs[blockIdx.y];
   __shared__ unsigned long long s_n[32];
   __shared__ unsigned s_t[32];
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -684,43 +708,71 @@ struct SortRows {
 
 // rows [b0, b0 + n), n <= kBucketCap, put in key order at the same place of
 // the output (which may be the input: every column is staged before it is written)
+template <bool K64, bool COL8>
 __device__ __forceinline__ void sort_bucket(const SortRows& s, unsigned char* sm, int64_t b0, int n) {
   const CtaOrder<kBucketCap, kBucketThreads, kBucketBins> c(sm);
   const int tid = threadIdx.x;
   for (int i = tid; i < n; i += kBucketThreads)
-    c.sk[i] = (s.key64 ? static_cast<const unsigned long long*>(s.keys)[b0 + i]
-                       : (unsigned long long)static_cast<const unsigned*>(s.keys)[b0 + i]) ^
+    c.sk[i] = (K64 ? static_cast<const unsigned long long*>(s.keys)[b0 + i]
+                   : (unsigned long long)static_cast<const unsigned*>(s.keys)[b0 + i]) ^
               s.flip;
   __syncthreads();
   c.run(n);
   for (int r = tid; r < n; r += kBucketThreads) {
     const unsigned long long k = c.sk[c.order[r]] ^ s.flip;
-    if (s.key64) static_cast<unsigned long long*>(s.okeys)[b0 + r] = k;
+    if (K64) static_cast<unsigned long long*>(s.okeys)[b0 + r] = k;
     else static_cast<unsigned*>(s.okeys)[b0 + r] = unsigned(k);
   }
   for (int a = 0; a < s.ncols; ++a) {
+    const void* col = s.cols[a];
+    void* ocol = s.ocols[a];
     __syncthreads();
     for (int i = tid; i < n; i += kBucketThreads)
-      c.sk[i] = s.col8 ? static_cast<const unsigned long long*>(s.cols[a])[b0 + i]
-                       : (unsigned long long)static_cast<const unsigned*>(s.cols[a])[b0 + i];
+      c.sk[i] = COL8 ? static_cast<const unsigned long long*>(col)[b0 + i]
+                     : (unsigned long long)static_cast<const unsigned*>(col)[b0 + i];
     __syncthreads();
     for (int r = tid; r < n; r += kBucketThreads) {
       const unsigned long long v = c.sk[c.order[r]];
-      if (s.col8) static_cast<unsigned long long*>(s.ocols[a])[b0 + r] = v;
-      else static_cast<unsigned*>(s.ocols[a])[b0 + r] = unsigned(v);
+      if (COL8) static_cast<unsigned long long*>(ocol)[b0 + r] = v;
+      else static_cast<unsigned*>(ocol)[b0 + r] = unsigned(v);
     }
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBucketThreads, 3) k_sort_buckets(SortRows s, const unsigned long long* offs, int nb,
-                                                                 const unsigned* fail) {
-  extern __shared__ __align__(16) unsigned char sm[];
-  if (*fail) return;
-  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
-    const unsigned long long lo = offs[b], hi = offs[b + 1];
-    if (hi > lo) sort_bucket(s, sm, int64_t(lo), int(hi - lo));
+// widths (compile time): dispatched once per CTA
+template <typename F>
+__device__ __forceinline__ void with_widths(const SortRows& s, F&& f) {
+  if (s.key64) {
+    if (s.col8) f(std::true_type{}, std::true_type{});
+    else f(std::true_type{}, std::false_type{});
+  } else {
+    if (s.col8) f(std::false_type{}, std::true_type{});
+    else f(std::false_type{}, std::false_type{});
   }
+}
+
+struct SortBucketArgs {
+  SortRows rows;
+  const unsigned long long* offs;
+  int nb;
+  const unsigned* fail;
+};
+
+__global__ void __launch_bounds__(kBucketThreads, 3) k_sort_buckets(const SortBucketArgs* jobs) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ __align__(8) SortBucketArgs s;
+  const unsigned* src = reinterpret_cast<const unsigned*>(jobs + blockIdx.y);
+  for (int w = threadIdx.x; w < int(sizeof(SortBucketArgs) / 4); w += kBucketThreads)
+    reinterpret_cast<unsigned*>(&s)[w] = src[w];
+  __syncthreads();
+  if (*s.fail) return;
+  with_widths(s.rows, [&](auto K, auto C) {
+    for (int b = blockIdx.x; b < s.nb; b += gridDim.x) {
+      const unsigned long long lo = s.offs[b], hi = s.offs[b + 1];
+      if (hi > lo) sort_bucket<decltype(K)::value, decltype(C)::value>(s.rows, sm, int64_t(lo), int(hi - lo));
+    }
+  });
 }
 
 // jobs of at most one bucket, one CTA each
@@ -730,7 +782,8 @@ __global__ void __launch_bounds__(kBucketThreads, 3) k_sort_small(const SortRows
   const unsigned* src = reinterpret_cast<const unsigned*>(jobs + blockIdx.x);
   for (int w = threadIdx.x; w < int(sizeof(SortRows) / 4); w += kBucketThreads) reinterpret_cast<unsigned*>(&s)[w] = src[w];
   __syncthreads();
-  sort_bucket(s, sm, 0, s.n);
+  if (s.key64) sort_bucket<true, true>(s, sm, 0, s.n);
+  else sort_bucket<false, true>(s, sm, 0, s.n);
 }
 
 __global__ void k_sort_iota(unsigned* idx, int64_t g) {
@@ -913,138 +966,242 @@ static bool sample_levels(int64_t g, int* b1, int* b2) {
   return true;
 }
 
-// Enqueues the sample sort of one job in the workspace at `base` (null: only
-// sizes it); *bytes: the workspace it takes.
-static gba_status sort_sample(gba_context* ctx, const SortJob& j, unsigned char* base, size_t* bytes, unsigned* d_fail,
-                              int* launches, cudaStream_t s) {
-  int b1 = 0, b2 = 0;
-  sample_levels(j.g, &b1, &b2);
-  const size_t np1 = size_t(1) << b1, np = size_t(1) << (b1 + b2), g = size_t(j.g);
-  // up to 4 aggregates travel with their key; more are gathered through the
-  // group's index afterwards
-  const bool direct = j.nagg <= GBA_MAX_COLS;
-  size_t o = 0;
+namespace {
+
+// One job of the sample sort: its shape and where its arrays are.
+struct SampleJob {
+  SortJob j;
+  int b1, b2;
+  bool direct;  // up to 4 aggregates travel with their key; more are gathered through the group's index
+  int nc;       // columns that travel
+  QDesc in;     // the level's input rows
+  int T[2], th[2];
+  size_t rows[2][1 + GBA_MAX_COLS];
+  size_t idx, idx_out, agg, hist[2], split[2], offs[2], cur[2], tiles;
+
+  size_t np(int x) const { return size_t(1) << (x ? b1 + b2 : b1); }
+};
+
+}  // namespace
+
+// Enqueues the sample sort of the jobs todo[first, last) in the workspace from
+// offset `front` on (dry: only sizes it); *bytes: the workspace they take.
+// Every step is one launch for all of them.
+static gba_status sort_sample(gba_context* ctx, const SortJob* jobs, const std::vector<int>& todo, size_t first,
+                              size_t last, size_t front, bool dry, size_t* bytes, unsigned* d_fail, int* launches,
+                              cudaStream_t s) {
+  std::vector<SampleJob> v(last - first);
+  const size_t nj = v.size();
+  size_t o = front;
   auto take = [&](size_t b) {
     const size_t at = o;
     o += a256(b);
     return at;
   };
-  const size_t kb = j.key64 ? 8 : 4, cb = direct ? 8 : 4;
-  const int nc = direct ? j.nagg : 1;
-  size_t rows[2][1 + GBA_MAX_COLS];
-  for (int x = 0; x < (b2 ? 2 : 1); ++x) {
-    rows[x][0] = take(g * kb);
-    for (int c = 0; c < nc; ++c) rows[x][1 + c] = take(g * cb);
+  // the counts come first: they are cleared together
+  for (size_t t = 0; t < nj; ++t) {
+    SampleJob& q = v[t];
+    q.j = jobs[todo[first + t]];
+    sample_levels(q.j.g, &q.b1, &q.b2);
+    q.direct = q.j.nagg <= GBA_MAX_COLS;
+    q.nc = q.direct ? q.j.nagg : 1;
+    q.hist[0] = take(8 * q.np(0));
+    q.hist[1] = q.b2 ? take(8 * q.np(1)) : 0;
   }
-  const size_t o_idx = direct ? 0 : take(g * 4), o_idx_out = direct ? 0 : take(g * 4);
-  const size_t o_agg = direct ? 0 : take(size_t(j.nagg) * a256(g * 8));
-  const size_t o_hist1 = take(8 * np1), o_hist2 = take(8 * np);  // cleared together
-  const size_t hist_bytes = o - o_hist1;
-  const size_t o_split1 = take(8 * np1), o_split2 = take(8 * np);
-  const size_t o_offs1 = take(8 * (np1 + 1)), o_offs2 = take(8 * (np + 1));
-  const size_t o_cur1 = take(8 * np1), o_cur2 = take(8 * np);
-  const size_t o_tiles = take(4 * (np1 + 1));
-  *bytes = o;
-  if (!base) return GBA_OK;
-  auto at = [&](size_t x) { return reinterpret_cast<unsigned long long*>(base + x); };
-  const unsigned long long flip = j.key_signed ? (j.key64 ? 1ull << 63 : 1ull << 31) : 0ull;
-  GBA_CUDA_TRY(ctx, cudaMemsetAsync(base + o_hist1, 0, hist_bytes, s));
+  const size_t hist_bytes = o - front;
+  for (SampleJob& q : v) {
+    const size_t g = size_t(q.j.g), kb = q.j.key64 ? 8 : 4, cb = q.direct ? 8 : 4;
+    for (int x = 0; x < (q.b2 ? 2 : 1); ++x) {
+      q.rows[x][0] = take(g * kb);
+      for (int c = 0; c < q.nc; ++c) q.rows[x][1 + c] = take(g * cb);
+      q.split[x] = take(8 * q.np(x));
+      q.offs[x] = take(8 * (q.np(x) + 1));
+      q.cur[x] = take(8 * q.np(x));
+    }
+    q.idx = q.direct ? 0 : take(g * 4);
+    q.idx_out = q.direct ? 0 : take(g * 4);
+    q.agg = q.direct ? 0 : take(size_t(q.j.nagg) * a256(g * 8));
+    q.tiles = take(4 * (q.np(0) + 1));
+  }
+  // argument arrays
+  const size_t o_args = o;
+  const size_t a_split = take(2 * nj * sizeof(SortSplitArgs)), a_hist = take(2 * nj * sizeof(SortHistArgs));
+  const size_t a_plan = take(2 * nj * sizeof(SortPlanArgs)), a_pass = take(2 * nj * sizeof(PartPass));
+  const size_t a_bucket = take(nj * sizeof(SortBucketArgs));
+  *bytes = o - front;
+  if (dry) return GBA_OK;
 
-  QDesc in{};
-  in.keys = j.keys;
-  in.n = j.g;
-  in.key64 = j.key64;
-  in.ncols = nc;
-  for (int c = 0; c < nc; ++c) {
-    in.col_type[c] = direct ? GBA_I64 : GBA_U32;
-    in.cols[c] = direct ? static_cast<const void*>(j.aggs[c]) : base + o_idx;
+  unsigned char* W = static_cast<unsigned char*>(ctx->ws);
+  auto at = [&](size_t x) { return reinterpret_cast<unsigned long long*>(W + x); };
+  std::vector<unsigned char> args(o - o_args);
+  auto arg = [&](size_t x) { return args.data() + (x - o_args); };
+  GBA_CUDA_TRY(ctx, cudaMemsetAsync(W + front, 0, hist_bytes, s));
+  auto wide_grid = [&](int64_t g) { return int(std::min<int64_t>(int64_t(ctx->sms) * 8, (g + 255) / 256)); };
+  for (SampleJob& q : v) {
+    q.in = QDesc{};
+    q.in.keys = q.j.keys;
+    q.in.n = q.j.g;
+    q.in.key64 = q.j.key64;
+    q.in.ncols = q.nc;
+    for (int c = 0; c < q.nc; ++c) {
+      q.in.col_type[c] = q.direct ? GBA_I64 : GBA_U32;
+      q.in.cols[c] = q.direct ? static_cast<const void*>(q.j.aggs[c]) : W + q.idx;
+    }
+    if (!q.direct) {
+      k_sort_iota<<<wide_grid(q.j.g), 256, 0, s>>>(reinterpret_cast<unsigned*>(W + q.idx), q.j.g);
+      GBA_CUDA_TRY(ctx, cudaGetLastError());
+      ++*launches;
+    }
   }
-  const int wide_grid = int(std::min<int64_t>(int64_t(ctx->sms) * 8, (j.g + 255) / 256));
-  if (!direct) {
-    k_sort_iota<<<wide_grid, 256, 0, s>>>(reinterpret_cast<unsigned*>(base + o_idx), j.g);
-    ++*launches;
+  // Per level: the jobs that have it, ordered so that one launch's scatter
+  // passes (key width, columns, CTA shape) are consecutive.
+  struct Pass {
+    size_t begin, end;
+    int64_t tiles;
+  };
+  std::vector<size_t> order[2];
+  std::vector<Pass> passes[2];
+  int64_t segs[2] = {1, 1}, tiles_most[2] = {0, 0};
+  for (int x = 0; x < 2; ++x) {
+    for (size_t t = 0; t < nj; ++t)
+      if (x == 0 || v[t].b2) order[x].push_back(t);
+    for (size_t t : order[x])
+      v[t].T[x] = gba_part_tile_rows(v[t].in, x ? v[t].b2 : v[t].b1, x ? int(v[t].np(0)) : 0, true, ctx->max_smem_optin,
+                                     &v[t].th[x]);
+    auto cls = [&](size_t t) { return (v[t].j.key64 * 8 + v[t].nc) * 2 + (v[t].th[x] == 1024) + (v[t].direct ? 0 : 64); };
+    std::stable_sort(order[x].begin(), order[x].end(), [&](size_t p, size_t q) { return cls(p) < cls(q); });
+    for (size_t i = 0; i < order[x].size(); ++i) {
+      const size_t t = order[x][i];
+      const int64_t tiles = v[t].j.g / v[t].T[x] + 1 + (x ? int64_t(v[t].np(0)) : 0);
+      if (i == 0 || cls(order[x][i - 1]) != cls(t)) passes[x].push_back(Pass{i, i, 0});
+      passes[x].back().end = i + 1;
+      passes[x].back().tiles = std::max(passes[x].back().tiles, tiles);
+      tiles_most[x] = std::max(tiles_most[x], tiles);
+      if (x) segs[1] = std::max<int64_t>(segs[1], int64_t(v[t].np(0)));
+    }
   }
-  int th[2] = {512, 512};
-  const int T1 = gba_part_tile_rows(in, b1, 0, true, ctx->max_smem_optin, &th[0]);
-  const int T2 = b2 ? gba_part_tile_rows(in, b2, int(np1), true, ctx->max_smem_optin, &th[1]) : 0;
-  for (int x = 0; x < (b2 ? 2 : 1); ++x) {
-    const int bits = x ? b2 : b1, nseg = x ? int(np1) : 0, T = x ? T2 : T1;
-    unsigned long long* split = at(x ? o_split2 : o_split1);
-    k_sort_split<<<x ? unsigned(np1) : 1u, kSampleThreads, order_smem(kSampleCap, kSampleBins), s>>>(
-        in.keys, j.key64, flip, j.g, x ? at(o_offs1) : nullptr, bits, split);
+  for (int x = 0; x < 2; ++x)
+    for (size_t i = 0; i < order[x].size(); ++i) {
+      const size_t t = order[x][i], slot = size_t(x) * nj + i;
+      SampleJob& q = v[t];
+      const unsigned long long flip = q.j.key_signed ? (q.j.key64 ? 1ull << 63 : 1ull << 31) : 0ull;
+      const int bits = x ? q.b2 : q.b1, nseg = x ? int(q.np(0)) : 0;
+      SortSplitArgs sp{};
+      sp.keys = q.in.keys;
+      sp.key64 = q.j.key64;
+      sp.flip = flip;
+      sp.n = q.j.g;
+      sp.bits = bits;
+      sp.nseg = nseg;
+      sp.offs = x ? at(q.offs[0]) : nullptr;
+      sp.split = at(q.split[x]);
+      SortHistArgs h{};
+      h.keys = q.in.keys;
+      h.key64 = q.j.key64;
+      h.flip = flip;
+      h.n = q.j.g;
+      h.bits = bits;
+      h.nseg = nseg;
+      h.T = q.T[x];
+      h.offs = sp.offs;
+      h.tile_prefix = reinterpret_cast<unsigned*>(W + q.tiles);
+      h.split = sp.split;
+      h.hist = at(q.hist[x]);
+      const bool ends = x || !q.b2;  // the level whose buckets are sorted in shared memory
+      SortPlanArgs pl{};
+      pl.np = int(q.np(x));
+      pl.hist = h.hist;
+      pl.offs = at(q.offs[x]);
+      pl.cursors = at(q.cur[x]);
+      pl.tile_prefix = ends ? nullptr : reinterpret_cast<unsigned*>(W + q.tiles);
+      pl.tile = ends ? 1 : q.T[1];
+      pl.cap = ends ? kBucketCap : 0;
+      pl.fail = d_fail + first + t;
+      PartPass pp{};
+      pp.in = q.in;
+      pp.out = q.in;
+      pp.out.keys = W + q.rows[x][0];
+      for (int c = 0; c < q.nc; ++c) pp.out.cols[c] = W + q.rows[x][1 + c];
+      pp.n = q.j.g;
+      pp.bits = bits;
+      pp.nseg = nseg;
+      pp.T = q.T[x];
+      pp.threads = q.th[x];
+      pp.offs = x ? at(q.offs[1]) : nullptr;
+      pp.tile_prefix = h.tile_prefix;
+      pp.cursors = pl.cursors;
+      pp.flags = reinterpret_cast<unsigned*>(ctx->d_small);
+      pp.splitters = sp.split;
+      pp.flip = flip;
+      pp.fail = pl.fail;
+      std::memcpy(arg(a_split) + slot * sizeof(sp), &sp, sizeof(sp));
+      std::memcpy(arg(a_hist) + slot * sizeof(h), &h, sizeof(h));
+      std::memcpy(arg(a_plan) + slot * sizeof(pl), &pl, sizeof(pl));
+      std::memcpy(arg(a_pass) + slot * sizeof(pp), &pp, sizeof(pp));
+      q.in = pp.out;
+      if (!ends) continue;
+      SortBucketArgs bk{};
+      bk.rows.keys = q.in.keys;
+      bk.rows.okeys = q.j.keys;
+      bk.rows.ncols = q.nc;
+      bk.rows.col8 = q.direct;
+      bk.rows.key64 = q.j.key64;
+      bk.rows.flip = flip;
+      for (int c = 0; c < q.nc; ++c) {
+        bk.rows.cols[c] = q.in.cols[c];
+        bk.rows.ocols[c] = q.direct ? static_cast<void*>(q.j.aggs[c]) : W + q.idx_out;
+      }
+      bk.offs = at(q.offs[x]);
+      bk.nb = int(q.np(x));
+      bk.fail = pl.fail;
+      std::memcpy(arg(a_bucket) + t * sizeof(bk), &bk, sizeof(bk));
+    }
+  GBA_CUDA_TRY(ctx, cudaMemcpyAsync(W + o_args, args.data(), args.size(), cudaMemcpyHostToDevice, s));
+  // CTAs per job: `most` over all jobs, each at least one
+  auto per_job = [&](int64_t want, int64_t most, size_t njobs) {
+    return unsigned(std::max<int64_t>(1, std::min<int64_t>(want, (most + int64_t(njobs) - 1) / int64_t(njobs))));
+  };
+  for (int x = 0; x < 2; ++x) {
+    const size_t n = order[x].size(), slot = size_t(x) * nj;
+    if (n == 0) continue;
+    k_sort_split<<<dim3(unsigned(segs[x]), unsigned(n)), kSampleThreads, order_smem(kSampleCap, kSampleBins), s>>>(
+        reinterpret_cast<const SortSplitArgs*>(W + a_split) + slot);
     GBA_CUDA_TRY(ctx, cudaGetLastError());
-    SortHistArgs h{};
-    h.keys = in.keys;
-    h.key64 = j.key64;
-    h.flip = flip;
-    h.n = j.g;
-    h.bits = bits;
-    h.nseg = nseg;
-    h.T = T;
-    h.offs = at(o_offs1);
-    h.tile_prefix = reinterpret_cast<unsigned*>(base + o_tiles);
-    h.split = split;
-    h.hist = at(x ? o_hist2 : o_hist1);
-    const int64_t tiles = j.g / T + 1 + nseg;
-    k_sort_hist<<<unsigned(std::min<int64_t>(tiles, int64_t(ctx->sms) * 4)), 512, 0, s>>>(h);
+    k_sort_hist<<<dim3(per_job(tiles_most[x], int64_t(ctx->sms) * 4, n), unsigned(n)), 512, 0, s>>>(
+        reinterpret_cast<const SortHistArgs*>(W + a_hist) + slot);
     GBA_CUDA_TRY(ctx, cudaGetLastError());
-    SortPlanArgs pl{};
-    pl.np = int(x ? np : np1);
-    pl.hist = h.hist;
-    pl.offs = at(x ? o_offs2 : o_offs1);
-    pl.cursors = at(x ? o_cur2 : o_cur1);
-    pl.tile_prefix = !x && b2 ? reinterpret_cast<unsigned*>(base + o_tiles) : nullptr;
-    pl.tile = !x && b2 ? T2 : 1;
-    pl.cap = x || !b2 ? kBucketCap : 0;
-    pl.fail = d_fail;
-    k_sort_plan<<<1, 1024, 0, s>>>(pl);
+    k_sort_plan<<<dim3(1, unsigned(n)), 1024, 0, s>>>(reinterpret_cast<const SortPlanArgs*>(W + a_plan) + slot);
     GBA_CUDA_TRY(ctx, cudaGetLastError());
-    PartPass pp{};
-    pp.in = in;
-    pp.out = in;
-    pp.out.keys = base + rows[x][0];
-    for (int c = 0; c < nc; ++c) pp.out.cols[c] = base + rows[x][1 + c];
-    pp.n = j.g;
-    pp.bits = bits;
-    pp.nseg = nseg;
-    pp.T = T;
-    pp.threads = th[x];
-    pp.offs = at(o_offs2);
-    pp.tile_prefix = h.tile_prefix;
-    pp.cursors = pl.cursors;
-    pp.flags = reinterpret_cast<unsigned*>(ctx->d_small);
-    pp.splitters = split;
-    pp.flip = flip;
-    pp.fail = d_fail;
-    GBA_CUDA_TRY(ctx, gba_launch_part_scatter(pp, int(std::min<int64_t>(tiles, ctx->sms * (1024 / th[x]))), s));
-    *launches += 4;
-    in = pp.out;
+    *launches += 3;
+    for (const Pass& p : passes[x]) {
+      const size_t np = p.end - p.begin;
+      const PartPass* host = reinterpret_cast<const PartPass*>(arg(a_pass)) + slot + p.begin;
+      GBA_CUDA_TRY(ctx, gba_launch_part_scatter_many(
+                            host, reinterpret_cast<const PartPass*>(W + a_pass) + slot + p.begin, int(np),
+                            int(per_job(p.tiles, int64_t(ctx->sms) * (1024 / host->threads), np)), s));
+      ++*launches;
+    }
   }
-  SortRows r{};
-  r.keys = in.keys;
-  r.okeys = j.keys;
-  r.ncols = nc;
-  r.col8 = direct;
-  r.key64 = j.key64;
-  r.flip = flip;
-  for (int c = 0; c < nc; ++c) {
-    r.cols[c] = in.cols[c];
-    r.ocols[c] = direct ? static_cast<void*>(j.aggs[c]) : base + o_idx_out;
-  }
-  k_sort_buckets<<<unsigned(std::min<int64_t>(int64_t(np), int64_t(ctx->sms) * 3)), kBucketThreads,
-                   order_smem(kBucketCap, kBucketBins), s>>>(r, at(b2 ? o_offs2 : o_offs1), int(np), d_fail);
+  int64_t nb_most = 1;
+  for (const SampleJob& q : v) nb_most = std::max<int64_t>(nb_most, int64_t(q.np(q.b2 ? 1 : 0)));
+  k_sort_buckets<<<dim3(per_job(nb_most, int64_t(ctx->sms) * 3, nj), unsigned(nj)), kBucketThreads,
+                   order_smem(kBucketCap, kBucketBins), s>>>(reinterpret_cast<const SortBucketArgs*>(W + a_bucket));
   GBA_CUDA_TRY(ctx, cudaGetLastError());
   ++*launches;
-  if (!direct) {
+  for (size_t t = 0; t < nj; ++t) {
+    const SampleJob& q = v[t];
+    if (q.direct) continue;
+    const size_t g = size_t(q.j.g);
     GatherCols c{};
-    c.n = j.nagg;
-    for (int a = 0; a < j.nagg; ++a) {
-      unsigned char* tmp = base + o_agg + size_t(a) * a256(g * 8);
-      GBA_CUDA_TRY(ctx, cudaMemcpyAsync(tmp, j.aggs[a], g * 8, cudaMemcpyDeviceToDevice, s));
+    c.n = q.j.nagg;
+    for (int a = 0; a < q.j.nagg; ++a) {
+      unsigned char* tmp = W + q.agg + size_t(a) * a256(g * 8);
+      GBA_CUDA_TRY(ctx, cudaMemcpyAsync(tmp, q.j.aggs[a], g * 8, cudaMemcpyDeviceToDevice, s));
       c.src[a] = reinterpret_cast<unsigned long long*>(tmp);
-      c.dst[a] = j.aggs[a];
+      c.dst[a] = q.j.aggs[a];
     }
-    k_sort_gather<<<wide_grid, kSortThreads, 0, s>>>(c, reinterpret_cast<unsigned*>(base + o_idx_out), j.g, d_fail);
+    k_sort_gather<<<wide_grid(q.j.g), kSortThreads, 0, s>>>(c, reinterpret_cast<unsigned*>(W + q.idx_out), q.j.g,
+                                                            d_fail + first + t);
     GBA_CUDA_TRY(ctx, cudaGetLastError());
     ++*launches;
   }
@@ -1062,17 +1219,29 @@ gba_status gba_sort_groups(gba_context* ctx, const SortJob* jobs, int njobs, cud
       return GBA_ERR_INVALID_ARG;
     }
     if (jobs[j].g <= kBucketCap) small.push_back(j);
-    else if (sample_levels(jobs[j].g, &b1, &b2)) {
-      size_t bytes;
-      int unused = 0;
-      sort_sample(ctx, jobs[j], nullptr, &bytes, nullptr, &unused, s);
-      most = std::max(most, bytes);
-      sample.push_back(j);
-    } else lsd.push_back(j);
+    else if (sample_levels(jobs[j].g, &b1, &b2)) sample.push_back(j);
+    else lsd.push_back(j);
+  }
+  // sampled jobs go together as long as 4 GiB of workspace hold them
+  std::vector<size_t> parts;  // first job of every part
+  size_t unused_bytes = 0;
+  int unused = 0;
+  for (size_t t = 0, sum = 0; t < sample.size(); ++t) {
+    sort_sample(ctx, jobs, sample, t, t + 1, 0, true, &unused_bytes, nullptr, &unused, s);
+    sum += unused_bytes;
+    if (t == 0 || sum > (size_t(4) << 30)) {
+      parts.push_back(t);
+      sum = unused_bytes;
+    }
+  }
+  for (size_t p = 0; p < parts.size(); ++p) {
+    sort_sample(ctx, jobs, sample, parts[p], p + 1 < parts.size() ? parts[p + 1] : sample.size(), 0, true, &unused_bytes,
+                nullptr, &unused, s);
+    most = std::max(most, unused_bytes);
   }
   if (!small.empty() || !sample.empty()) {
     // front of the workspace: the small jobs' descriptors, then one failure
-    // word per sampled job (they share the rest, one after another)
+    // word per sampled job (their parts share the rest, one after another)
     const size_t o_fail = a256(small.size() * sizeof(SortRows)), front = o_fail + a256(4 * sample.size() + 4);
     gba_status st = gba_ws_reserve(ctx, front + most, s);
     if (st != GBA_OK) return st;
@@ -1110,9 +1279,9 @@ gba_status gba_sort_groups(gba_context* ctx, const SortJob* jobs, int njobs, cud
     }
     if (!sample.empty()) {
       GBA_CUDA_TRY(ctx, cudaMemsetAsync(d_fail, 0, 4 * sample.size(), s));
-      for (size_t t = 0; t < sample.size(); ++t) {
-        size_t bytes;
-        st = sort_sample(ctx, jobs[sample[t]], W + front, &bytes, d_fail + t, &launches, s);
+      for (size_t p = 0; p < parts.size(); ++p) {
+        st = sort_sample(ctx, jobs, sample, parts[p], p + 1 < parts.size() ? parts[p + 1] : sample.size(), front, false,
+                         &unused_bytes, d_fail, &launches, s);
         if (st != GBA_OK) return st;
       }
       GBA_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_small + 64, d_fail, 4 * sample.size(), cudaMemcpyDeviceToHost, s));

@@ -83,4 +83,7 @@ cudaError_t gba_launch_part_hist(const QDesc& q, int bits, unsigned long long* h
                                  cudaStream_t s);
 cudaError_t gba_launch_part_plan(const PartPlanArgs& a, cudaStream_t s);
 cudaError_t gba_launch_part_scatter(const PartPass& p, int grid, cudaStream_t s);
+// n passes by key range (splitters set), of one key width, column count and
+// CTA shape, in one launch of `grid` CTAs each; host and device: the same array
+cudaError_t gba_launch_part_scatter_many(const PartPass* host, const PartPass* device, int n, int grid, cudaStream_t s);
 cudaError_t gba_launch_part_agg(const PartAgg& a, int ctas, int grid, cudaStream_t s);

@@ -67,3 +67,26 @@ def test_sorted_past_two_levels(ctx):
     assert res.n_groups == n
     assert torch.equal(res.keys, torch.sort(keys).values)
     assert bool((res.aggs[0] == 1).all())
+
+
+def test_sorted_batch_of_mixed_jobs(ctx):
+    """One call whose queries take every route of the sort: empty, one bucket,
+    one and two levels, both key widths, 1 to 5 aggregates."""
+    from gpu_util import to_device
+    rng = np.random.default_rng(4)
+    aggs = [("sum", 0), ("count", None), ("max", 0), ("min", 0), ("max", 0)]
+    specs = [(1, 1), (5000, 1), (4096, 2), (4097, 2), (30_000, 4), (30_000, 5), (400_003, 2), (400_003, 3), (9000, 1)]
+    host, qs = [], []
+    for i, (n, na) in enumerate(specs):
+        kdt = (np.int64, np.int32, np.uint32)[i % 3]
+        keys, cols = _keys("uniform", n, np.int64 if kdt == np.int64 else np.int32, rng).astype(kdt), \
+            [rng.integers(-1000, 1000, size=n)]
+        host.append((keys, cols, aggs[:na]))
+        qs.append((to_device(keys), [to_device(cols[0])], aggs[:na], kdt == np.uint32))
+    for (keys, cols, a), r in zip(host, ctx.groupby_batch(qs, knobs=dict(sort_output=1))):
+        gk = r.keys.cpu().numpy()
+        gk = gk.view(np.uint32) if keys.dtype == np.uint32 else gk
+        ok, oa = O.groupby(keys, cols, a, nthreads=8)
+        np.testing.assert_array_equal(gk, ok)
+        for g, o in zip(r.aggs, oa):
+            np.testing.assert_array_equal(g.cpu().numpy(), o)
