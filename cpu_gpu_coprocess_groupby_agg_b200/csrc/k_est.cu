@@ -107,7 +107,7 @@ __device__ __noinline__ unsigned long long est_count_insert(unsigned long long* 
   return 0ull;  // unreachable: the table holds 1.5x the sample
 }
 
-// One block per chunk of GBA_EST_CHUNK_TILES sampled tiles of one query (a
+// One block per chunk of chunk_tiles sampled tiles of one query (a
 // flat grid over every query's chunks).  Per sampled row: the 64 HLL
 // registers (block-local, merged once), and the query's count table (keys +
 // counts, linear probing, capacity 1.5x the sample).  Lanes of a warp
@@ -117,7 +117,7 @@ __device__ __noinline__ unsigned long long est_count_insert(unsigned long long* 
 // step's loads and atomics issued before any result is used.
 constexpr int kEstThreads = 256;
 constexpr int kEstU = 4;
-__global__ void __launch_bounds__(kEstThreads) k_est_sample(const EstQuery* qs, int nq) {
+__global__ void __launch_bounds__(kEstThreads) k_est_sample(const EstQuery* qs, int nq, int chunk_tiles) {
   __shared__ unsigned long long sf[7];
   __shared__ unsigned s_hll[64];
   int lo = 0, hi = nq - 1;
@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(kEstThreads) k_est_sample(const EstQuery* qs, 
   if (threadIdx.x < 64) s_hll[threadIdx.x] = 0u;
   __syncthreads();
   const int64_t items = int64_t(e.sampled_tiles) << 10;
-  const int64_t c0 = chunk * (int64_t(GBA_EST_CHUNK_TILES) << 10);
-  const int64_t c1 = c0 + (int64_t(GBA_EST_CHUNK_TILES) << 10) < items ? c0 + (int64_t(GBA_EST_CHUNK_TILES) << 10) : items;
+  const int64_t c0 = chunk * (int64_t(chunk_tiles) << 10);
+  const int64_t c1 = c0 + (int64_t(chunk_tiles) << 10) < items ? c0 + (int64_t(chunk_tiles) << 10) : items;
   FreqAcc f;
 #pragma unroll
   for (int c = 0; c < 5; ++c) f.d[c] = 0;
@@ -443,13 +443,13 @@ size_t train_smem() { return sizeof(float) * (size_t(kTrainB) * (F + 5 * H) + kT
 
 // ---------------------------------------------------------------------------
 // launchers
-cudaError_t gba_launch_est_sample(const EstQuery* d_qs, int nq, int64_t total_chunks, cudaStream_t s) {
-  // a flat grid: one block per chunk of GBA_EST_CHUNK_TILES sampled tiles of
+cudaError_t gba_launch_est_sample(const EstQuery* d_qs, int nq, int64_t total_chunks, int chunk_tiles, cudaStream_t s) {
+  // a flat grid: one block per chunk of chunk_tiles sampled tiles of
   // a query, so every query gets as many blocks as its sample needs (a grid
   // of queries x the largest query's blocks left most blocks empty)
   if (nq <= 0 || total_chunks <= 0) return cudaSuccess;
   if (total_chunks > int64_t(0x7fffffff)) return cudaErrorInvalidValue;
-  k_est_sample<<<unsigned(total_chunks), kEstThreads, 0, s>>>(d_qs, nq);
+  k_est_sample<<<unsigned(total_chunks), kEstThreads, 0, s>>>(d_qs, nq, chunk_tiles);
   return cudaGetLastError();
 }
 cudaError_t gba_launch_est_init(const EstQuery* d_qs, int nq, cudaStream_t s) {
@@ -649,12 +649,20 @@ gba_status gba_est_features_device(gba_context* ctx, const QDesc* qs, int nq, in
   const size_t o_h = take(4 * 64 * size_t(nq));
   const size_t o_fr = take(8 * 8 * size_t(nq));
   std::vector<size_t> o_t(nq);
-  int64_t chunks = 0;
+  int64_t chunks = 0, tiles = 0;
   for (int i = 0; i < nq; ++i) {
     gba_est_plan(&eq[i], qs[i].n, tile_rows);
     o_t[i] = take(16 * eq[i].cap);
+    tiles += eq[i].sampled_tiles;
+  }
+  // A block's tiles are a chain of dependent round trips, so few tiles get a
+  // block each; many share one, whose sums they add to the query's once (us, 4
+  // tiles a block against 1: one large query 160 / 66, 48 small ones 73 / 43,
+  // 256 mixed ones with 9652 tiles 340 / 536).
+  const int chunk_tiles = tiles <= int64_t(ctx->sms) * 16 ? 1 : 4;
+  for (int i = 0; i < nq; ++i) {
     eq[i].chunk_base = chunks;
-    eq[i].nchunks = (eq[i].sampled_tiles + GBA_EST_CHUNK_TILES - 1) / GBA_EST_CHUNK_TILES;
+    eq[i].nchunks = (eq[i].sampled_tiles + chunk_tiles - 1) / chunk_tiles;
     chunks += eq[i].nchunks;
   }
   gba_status st = gba_est_reserve(ctx, off, s);
@@ -675,7 +683,7 @@ gba_status gba_est_features_device(gba_context* ctx, const QDesc* qs, int nq, in
   GBA_CUDA_TRY(ctx, cudaMemcpyAsync(base + o_q, eq.data(), sizeof(EstQuery) * nq, cudaMemcpyHostToDevice, s));
   const EstQuery* dq = reinterpret_cast<const EstQuery*>(base + o_q);
   GBA_CUDA_TRY(ctx, gba_launch_est_init(dq, nq, s));
-  GBA_CUDA_TRY(ctx, gba_launch_est_sample(dq, nq, chunks, s));
+  GBA_CUDA_TRY(ctx, gba_launch_est_sample(dq, nq, chunks, chunk_tiles, s));
   GBA_CUDA_TRY(ctx, gba_launch_est_reduce(dq, nq, s));
   *feats_out = reinterpret_cast<float*>(base + o_f);
   *stats_out = reinterpret_cast<unsigned long long*>(base + o_s);
