@@ -15,8 +15,9 @@
 //   k_sort_plan     bucket bounds, write cursors, tiles of the next level
 //   k_part_scatter  (k_part.cu) keys and aggregate columns moved to their buckets
 //   k_sort_buckets  a CTA orders one bucket in shared memory and writes its keys
-//                   and aggregates to their final place
-// One level for up to 2^19 groups, two levels above.  Jobs of up to one bucket
+//                   and aggregates to their final place (k_sort_big_buckets:
+//                   the few buckets of two-level jobs of twice the size)
+// One level for up to 2^18 groups, two levels above.  Jobs of up to one bucket
 // are all sorted in place by one launch (k_sort_small).
 //
 // Bytes per group of b bytes: 2 (b + key) per level and 2 b for the buckets,
@@ -527,6 +528,7 @@ struct SortSplitArgs {
   unsigned long long flip;
   int64_t n;
   int bits, nseg;                  // nseg = 0: one segment [0, n)
+  int sample;                      // keys to sample (at most kSampleCap)
   const unsigned long long* offs;  // segment bounds
   unsigned long long* split;       // [segment][2^bits]
 };
@@ -545,8 +547,7 @@ __global__ void __launch_bounds__(kSampleThreads) k_sort_split(const SortSplitAr
   const CtaOrder<kSampleCap, kSampleThreads, kSampleBins> s(sm);
   const int64_t b = offs ? int64_t(offs[blockIdx.x]) : 0, e = offs ? int64_t(offs[blockIdx.x + 1]) : n;
   const int64_t rows = e - b;
-  const int want = kSamplePer << bits < kSampleCap ? kSamplePer << bits : kSampleCap;
-  const int m = int(rows < want ? rows : want);
+  const int m = int(rows < a.sample ? rows : a.sample);
   for (int i = threadIdx.x; i < m; i += kSampleThreads) s.sk[i] = sort_key(keys, key64, b + rows * i / m, flip);
   __syncthreads();
   s.run(m);
@@ -706,19 +707,19 @@ struct SortRows {
   unsigned long long flip;
 };
 
-// rows [b0, b0 + n), n <= kBucketCap, put in key order at the same place of
+// rows [b0, b0 + n), n <= CAP, put in key order at the same place of
 // the output (which may be the input: every column is staged before it is written)
-template <bool K64, bool COL8>
+template <bool K64, bool COL8, int CAP = kBucketCap, int THREADS = kBucketThreads, int BINS = kBucketBins>
 __device__ __forceinline__ void sort_bucket(const SortRows& s, unsigned char* sm, int64_t b0, int n) {
-  const CtaOrder<kBucketCap, kBucketThreads, kBucketBins> c(sm);
+  const CtaOrder<CAP, THREADS, BINS> c(sm);
   const int tid = threadIdx.x;
-  for (int i = tid; i < n; i += kBucketThreads)
+  for (int i = tid; i < n; i += THREADS)
     c.sk[i] = (K64 ? static_cast<const unsigned long long*>(s.keys)[b0 + i]
                    : (unsigned long long)static_cast<const unsigned*>(s.keys)[b0 + i]) ^
               s.flip;
   __syncthreads();
   c.run(n);
-  for (int r = tid; r < n; r += kBucketThreads) {
+  for (int r = tid; r < n; r += THREADS) {
     const unsigned long long k = c.sk[c.order[r]] ^ s.flip;
     if (K64) static_cast<unsigned long long*>(s.okeys)[b0 + r] = k;
     else static_cast<unsigned*>(s.okeys)[b0 + r] = unsigned(k);
@@ -727,11 +728,11 @@ __device__ __forceinline__ void sort_bucket(const SortRows& s, unsigned char* sm
     const void* col = s.cols[a];
     void* ocol = s.ocols[a];
     __syncthreads();
-    for (int i = tid; i < n; i += kBucketThreads)
+    for (int i = tid; i < n; i += THREADS)
       c.sk[i] = COL8 ? static_cast<const unsigned long long*>(col)[b0 + i]
                      : (unsigned long long)static_cast<const unsigned*>(col)[b0 + i];
     __syncthreads();
-    for (int r = tid; r < n; r += kBucketThreads) {
+    for (int r = tid; r < n; r += THREADS) {
       const unsigned long long v = c.sk[c.order[r]];
       if (COL8) static_cast<unsigned long long*>(ocol)[b0 + r] = v;
       else static_cast<unsigned*>(ocol)[b0 + r] = unsigned(v);
@@ -770,9 +771,36 @@ __global__ void __launch_bounds__(kBucketThreads, 3) k_sort_buckets(const SortBu
   with_widths(s.rows, [&](auto K, auto C) {
     for (int b = blockIdx.x; b < s.nb; b += gridDim.x) {
       const unsigned long long lo = s.offs[b], hi = s.offs[b + 1];
-      if (hi > lo) sort_bucket<decltype(K)::value, decltype(C)::value>(s.rows, sm, int64_t(lo), int(hi - lo));
+      if (hi > lo && hi - lo <= kBucketCap)
+        sort_bucket<decltype(K)::value, decltype(C)::value>(s.rows, sm, int64_t(lo), int(hi - lo));
     }
   });
+}
+
+// the rare buckets of two-level jobs that are larger than kBucketCap
+__global__ void __launch_bounds__(kSampleThreads) k_sort_big_buckets(const SortBucketArgs* jobs) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ int s_big[kSampleThreads];
+  __shared__ int s_n;
+  const SortBucketArgs& s = jobs[blockIdx.y];
+  if (*s.fail) return;
+  // a thread looks at one bucket: the few large ones are listed, then sorted
+  for (int base = int(blockIdx.x) * kSampleThreads; base < s.nb; base += int(gridDim.x) * kSampleThreads) {
+    const int b = base + int(threadIdx.x);
+    const bool big = b < s.nb && s.offs[b + 1] - s.offs[b] > kBucketCap;
+    if (threadIdx.x == 0) s_n = 0;
+    if (!__syncthreads_or(big)) continue;
+    if (big) s_big[atomicAdd(&s_n, 1)] = b;
+    __syncthreads();
+    for (int i = 0; i < s_n; ++i) {
+      const unsigned long long lo = s.offs[s_big[i]], hi = s.offs[s_big[i] + 1];
+      with_widths(s.rows, [&](auto K, auto C) {
+        sort_bucket<decltype(K)::value, decltype(C)::value, kSampleCap, kSampleThreads, kSampleBins>(
+            s.rows, sm, int64_t(lo), int(hi - lo));
+      });
+    }
+    __syncthreads();
+  }
 }
 
 // jobs of at most one bucket, one CTA each
@@ -949,9 +977,12 @@ static gba_status sort_lsd(gba_context* ctx, const SortJob* jobs, const std::vec
 }
 
 // Splitter bits of a job's two levels (b2 = 0: one level); false: too many
-// groups for them.  64 sampled keys per bucket keep a bucket under twice its
-// mean (chance of one that is not: 3e-9); at 8 bits a level, 32 samples, the
-// mean is at most a third of what a bucket may hold.
+// groups for them.  A bucket of s sampled keys outgrows x times its mean with a
+// chance of about exp(-s (x - 1 - ln x)).  One level: s = 64, x = 2, 3e-9.  Two:
+// a first-level segment of 128 sampled keys may be 1.27 times its mean, so a few
+// buckets in 10^4 pass kBucketCap (k_sort_big_buckets takes them), and none
+// twice that: x = 3, 1e-25.  At 8 bits a level (s = 32, segments up to 1.53
+// times their mean, a mean of a third of kBucketCap) x = 4, 1e-22.
 static bool sample_levels(int64_t g, int* b1, int* b2) {
   auto bits_for = [&](int64_t per) {
     int b = 1;
@@ -959,9 +990,14 @@ static bool sample_levels(int64_t g, int* b1, int* b2) {
     return b;
   };
   int b = bits_for(kBucketTarget);
+  if (b <= kLevelBits - 1) {
+    *b1 = b;
+    *b2 = 0;
+    return true;
+  }
   if (b > 2 * (kLevelBits - 1)) b = bits_for(kBucketCap / 3);
   if (b > 2 * kLevelBits) return false;
-  *b1 = b <= kLevelBits - 1 ? b : b / 2;
+  *b1 = b / 2;
   *b2 = b - *b1;
   return true;
 }
@@ -1093,6 +1129,7 @@ static gba_status sort_sample(gba_context* ctx, const SortJob* jobs, const std::
       sp.n = q.j.g;
       sp.bits = bits;
       sp.nseg = nseg;
+      sp.sample = x == 0 && q.b2 ? kSampleCap : std::min(kSamplePer << bits, kSampleCap);
       sp.offs = x ? at(q.offs[0]) : nullptr;
       sp.split = at(q.split[x]);
       SortHistArgs h{};
@@ -1115,7 +1152,7 @@ static gba_status sort_sample(gba_context* ctx, const SortJob* jobs, const std::
       pl.cursors = at(q.cur[x]);
       pl.tile_prefix = ends ? nullptr : reinterpret_cast<unsigned*>(W + q.tiles);
       pl.tile = ends ? 1 : q.T[1];
-      pl.cap = ends ? kBucketCap : 0;
+      pl.cap = !ends ? 0 : x ? kSampleCap : kBucketCap;
       pl.fail = d_fail + first + t;
       PartPass pp{};
       pp.in = q.in;
@@ -1188,6 +1225,12 @@ static gba_status sort_sample(gba_context* ctx, const SortJob* jobs, const std::
                    order_smem(kBucketCap, kBucketBins), s>>>(reinterpret_cast<const SortBucketArgs*>(W + a_bucket));
   GBA_CUDA_TRY(ctx, cudaGetLastError());
   ++*launches;
+  if (!order[1].empty()) {
+    k_sort_big_buckets<<<dim3(per_job(nb_most, ctx->sms, nj), unsigned(nj)), kSampleThreads,
+                         order_smem(kSampleCap, kSampleBins), s>>>(reinterpret_cast<const SortBucketArgs*>(W + a_bucket));
+    GBA_CUDA_TRY(ctx, cudaGetLastError());
+    ++*launches;
+  }
   for (size_t t = 0; t < nj; ++t) {
     const SampleJob& q = v[t];
     if (q.direct) continue;
@@ -1250,6 +1293,7 @@ gba_status gba_sort_groups(gba_context* ctx, const SortJob* jobs, int njobs, cud
     static const cudaError_t smem_ok = [] {
       cudaError_t e = gba_allow_max_smem(k_sort_split);
       if (e == cudaSuccess) e = gba_allow_max_smem(k_sort_buckets);
+      if (e == cudaSuccess) e = gba_allow_max_smem(k_sort_big_buckets);
       return e != cudaSuccess ? e : gba_allow_max_smem(k_sort_small);
     }();
     GBA_CUDA_TRY(ctx, smem_ok);
