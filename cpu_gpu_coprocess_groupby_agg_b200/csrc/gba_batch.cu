@@ -11,8 +11,9 @@
 // replayed from a CUDA graph while the batch's launch shapes repeat (the
 // per-query descriptors are copied from pinned host memory by the graph's
 // first node, so new queries of the same shapes reuse it).  Queries on the
-// partition strategy run one after another behind it.  A query whose table
-// overflowed is rerun alone with a larger table.
+// partition strategy are enqueued one after another before it, and all are
+// waited for once.  A query whose table overflowed is rerun alone with a larger
+// table.
 //
 // No counterpart in the reference: its host loop runs one query, one tile per
 // stream at a time (group_then_partition.cu:332-424).
@@ -177,8 +178,8 @@ static gba_status batch_avg(gba_context* ctx, int32_t nq, const gba_query* qs, c
                             const gba_knobs* knobs, void* stream, int64_t* n_groups);
 
 // Composite keys are packed into 64-bit keys around the batch; key order
-// (knobs->sort_output) sorts every query's groups on the device after it, one
-// query after another.
+// (knobs->sort_output) sorts every query's groups on the device after it, each
+// step of the sort one launch for all queries.
 extern "C" gba_status gba_groupby_batch(gba_context* ctx, int32_t nq, const gba_query* qs, const gba_output* outs,
                                         const gba_knobs* knobs, void* stream, int64_t* n_groups) {
   if (!ctx || nq < 0 || (nq > 0 && (!qs || !outs || !n_groups))) return GBA_ERR_INVALID_ARG;

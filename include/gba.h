@@ -105,7 +105,8 @@ typedef struct gba_output {
 } gba_output;
 
 typedef enum gba_sizing {
-  GBA_SIZING_PLAIN = 0,   /* fixed load factor on the row count, overflow -> regrow */
+  GBA_SIZING_PLAIN = 0,   /* fixed load factor on the row count, overflow -> regrow; a single query of more than
+                             2^20 rows (AUTO strategy) by a sample of its rows */
   GBA_SIZING_LEARNED = 1, /* MLP cardinality estimate, overflow -> regrow */
   GBA_SIZING_FIXED = 2,   /* table_slots as given, overflow -> regrow */
   GBA_SIZING_GROW = 3     /* estimator-free: the plain capacity, but at most table_slots (default 2^16)
